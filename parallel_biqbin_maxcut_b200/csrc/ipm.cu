@@ -22,7 +22,6 @@
 // pivot is exactly "Z not positive definite".
 #include "ipm.cuh"
 #include "cta_linalg.cuh"
-#include "reg_linalg.cuh"
 #include "ipm_reg_body.cuh"
 
 #include <math.h>
@@ -279,20 +278,18 @@ __device__ void ipm_body(const IpmDesc& d, double* smem, int place)
 }
 
 __global__ void __launch_bounds__(IPM_THREADS, 1)
-ipm_reg_one_kernel(IpmDesc d, int zi_in_smem)
+ipm_reg_one_kernel(IpmDesc d, int smem_doubles)
 {
-    extern __shared__ __align__(16) double smem[];
     if (d.n <= 0) return;
-    ipm_body_reg(d, smem, zi_in_smem, g_ipm_stats);
+    ipm_body_reg(d, smem_doubles, g_ipm_stats);
 }
 
 __global__ void __launch_bounds__(IPM_THREADS, 1)
-ipm_reg_batched_kernel(const IpmDesc* __restrict__ descs, int zi_in_smem)
+ipm_reg_batched_kernel(const IpmDesc* __restrict__ descs, int smem_doubles)
 {
-    extern __shared__ __align__(16) double smem[];
     const IpmDesc d = descs[blockIdx.x];
     if (d.n <= 0) return;
-    ipm_body_reg(d, smem, zi_in_smem, g_ipm_stats);
+    ipm_body_reg(d, smem_doubles, g_ipm_stats);
 }
 
 __global__ void __launch_bounds__(IPM_THREADS, 1)
@@ -300,14 +297,6 @@ ipm_batched_kernel(const IpmDesc* __restrict__ descs, int place)
 {
     extern __shared__ __align__(16) double smem[];
     const IpmDesc d = descs[blockIdx.x];
-    if (d.n <= 0) return;
-    ipm_body(d, smem, place);
-}
-
-__global__ void __launch_bounds__(IPM_THREADS, 1)
-ipm_one_kernel(IpmDesc d, int place)
-{
-    extern __shared__ __align__(16) double smem[];
     if (d.n <= 0) return;
     ipm_body(d, smem, place);
 }
@@ -334,10 +323,10 @@ int ipm_place(int n_max, size_t smem_limit, size_t* smem_bytes)
 size_t ipm_ws_doubles(int n, int place)
 {
     const size_t nn = (size_t)n * n;
-    return nn * (2 + ((place & 1) ? 0 : 1) + ((place & 2) ? 0 : 1));
+    const size_t staged = nn * (2 + ((place & 1) ? 0 : 1) + ((place & 2) ? 0 : 1));
+    const size_t tiles = n <= ST_NMAX ? ipm_st_ws_doubles(n) : 0;
+    return ((staged > tiles ? staged : tiles) + 1) & ~(size_t)1;   // (tile pairs are 16-byte accesses)
 }
-
-
 
 // Optional CUDA-event timing of every IPM launch on its stream (for the
 // benchmark's per-kernel roofline figure).  Each host thread records its
@@ -418,28 +407,21 @@ struct IpmThreadTimer {
 };
 static thread_local IpmThreadTimer t_timer;
 
-// Register path (n <= 128): F always in shared memory; Zi too when it fits.
-// Its fixed shared-memory part is smaller than the staged path's
-// (ipm_fixed_smem_doubles), so whenever ipm_place puts both matrices in
-// shared memory this path does too, and the workspace ipm_ws_doubles gives
-// for ipm_place's placement always covers it (2 or 3 n^2 doubles).
-static int ipm_reg_place(int n_max, size_t smem_limit, size_t* smem_bytes)
+// Shared memory of the n <= 128 kernels, in doubles.
+static int ipm_reg_smem(int n_max)
 {
-    const size_t fixed = ipm_reg_fixed_smem_doubles(n_max) * sizeof(double);
-    const size_t mat = (size_t)n_max * n_max * sizeof(double);
-    const int zi = fixed + 2 * mat <= smem_limit ? 1 : 0;
-    *smem_bytes = fixed + (zi ? 2 : 1) * mat;
-    return zi;
+    return (int)ipm_st_smem_doubles_upto(n_max, rt().smem_optin / sizeof(double));
 }
 
 void ipm_launch(const IpmDesc* d_descs, int nprob, int n_max, cudaStream_t s)
 {
     if (nprob <= 0) return;
     size_t bytes = 0;
-    if (n_max <= RM_NMAX) {
-        const int zi = ipm_reg_place(n_max, rt().smem_optin, &bytes);
+    if (n_max <= ST_NMAX) {
+        const int sd = ipm_reg_smem(n_max);
+        bytes = sd * sizeof(double);
         BQB_SMEM_LIMIT(ipm_reg_batched_kernel, bytes);
-        t_timer.timed(s, [&] { ipm_reg_batched_kernel<<<nprob, IPM_THREADS, bytes, s>>>(d_descs, zi); });
+        t_timer.timed(s, [&] { ipm_reg_batched_kernel<<<nprob, IPM_THREADS, bytes, s>>>(d_descs, sd); });
         BQB_COUNT_LAUNCH();
         check_launch("ipm_reg_batched_kernel");
         return;
@@ -454,28 +436,27 @@ void ipm_launch(const IpmDesc* d_descs, int nprob, int n_max, cudaStream_t s)
 void ipm_launch_one(const IpmDesc& d, cudaStream_t s)
 {
     size_t bytes = 0;
-    if (d.n <= RM_NMAX) {
-        const int zi = ipm_reg_place(d.n, rt().smem_optin, &bytes);
+    if (d.n <= ST_NMAX) {
+        const int sd = ipm_reg_smem(d.n);
+        bytes = sd * sizeof(double);
         BQB_SMEM_LIMIT(ipm_reg_one_kernel, bytes);
-        t_timer.timed(s, [&] { ipm_reg_one_kernel<<<1, IPM_THREADS, bytes, s>>>(d, zi); });
+        t_timer.timed(s, [&] { ipm_reg_one_kernel<<<1, IPM_THREADS, bytes, s>>>(d, sd); });
         BQB_COUNT_LAUNCH();
         check_launch("ipm_reg_one_kernel");
         return;
     }
-    const int place = ipm_place(d.n, rt().smem_optin, &bytes);
-    BQB_SMEM_LIMIT(ipm_one_kernel, bytes);
-    t_timer.timed(s, [&] { ipm_one_kernel<<<1, IPM_THREADS, bytes, s>>>(d, place); });
-    BQB_COUNT_LAUNCH();
-    check_launch("ipm_one_kernel");
+    fatal("ipm_launch_one", "n above the one-CTA limit");   // (ipm_device sends those to ipm_large)
 }
 
 // Single-problem launch for callers that manage the scratch (d.ws) and the
-// placement themselves; records no timing events and allocates nothing.
-cudaError_t ipm_launch_prepared(const IpmDesc& d, int place, size_t smem_bytes, cudaStream_t s)
+// shared-memory limit themselves; records no timing events and allocates
+// nothing.
+cudaError_t ipm_launch_prepared(const IpmDesc& d, size_t smem_limit, cudaStream_t s)
 {
-    cudaError_t e = raise_smem_limit((const void*)ipm_one_kernel, smem_bytes);
+    const size_t sd = ipm_st_smem_doubles(d.n, smem_limit / sizeof(double));
+    cudaError_t e = raise_smem_limit((const void*)ipm_reg_one_kernel, sd * sizeof(double));
     if (e != cudaSuccess) return e;
-    ipm_one_kernel<<<1, IPM_THREADS, smem_bytes, s>>>(d, place);
+    ipm_reg_one_kernel<<<1, IPM_THREADS, sd * sizeof(double), s>>>(d, (int)sd);
     BQB_COUNT_LAUNCH();
     return cudaGetLastError();
 }

@@ -44,11 +44,11 @@ size_t ipm_ws_doubles(int n, int place);
 
 // Launch the batched kernel over `nprob` descriptors already on the device.
 void ipm_launch(const IpmDesc* d_descs, int nprob, int n_max, cudaStream_t s);
-// Single problem: descriptor passed by value.
+// Single problem (n <= 128): descriptor passed by value.
 void ipm_launch_one(const IpmDesc& d, cudaStream_t s);
-// Single problem with placement chosen by the caller; returns the launch
-// status instead of raising it.
-cudaError_t ipm_launch_prepared(const IpmDesc& d, int place, size_t smem_bytes, cudaStream_t s);
+// Single problem (n <= 128) on a device with smem_limit bytes of opt-in
+// shared memory; returns the launch status instead of raising it.
+cudaError_t ipm_launch_prepared(const IpmDesc& d, size_t smem_limit, cudaStream_t s);
 
 // Device address of the IPM work counters (for kernels in other files that
 // run the IPM body).

@@ -11,10 +11,9 @@
 //
 // Limits and rules:
 //  * n <= BQB_IPM_NOALLOC_NMAX (128).  The scratch array holds 3 * 128^2
-//    doubles (384 KiB): the IPM keeps dX and dX1 in global memory, plus Zi
-//    when only the Cholesky workspace fits in shared memory (n > 118).
-//    Every GPU that loads the library holds this array until the process
-//    exits.
+//    doubles (384 KiB), of which the IPM uses at most 25,088: dX / dX1 and the
+//    inverse of M where they do not fit in shared memory.  Every GPU that
+//    loads the library holds this array until the process exits.
 //  * The first call on a device resolves the array's device address
 //    (cudaGetSymbolAddress, with that device current) and caches it; make
 //    that first call before any stream capture.
@@ -86,14 +85,13 @@ extern "C" __attribute__((visibility("default"))) int bqb_ipm_noalloc(const doub
         ws = g_scratch_ptr[dev];
         optin = g_smem_optin[dev];
     }
-    size_t bytes = 0;
-    const int place = bqb::ipm_place(n, optin, &bytes);
+    const int place = bqb::ipm_place(n, optin, nullptr);
     if (bqb::ipm_ws_doubles(n, place) > NOALLOC_DOUBLES) {
         bqb::set_error("bqb_ipm_noalloc", "scratch too small for this placement");
         return 1;
     }
     const bqb::IpmDesc d{L, X, ws, out, nullptr, n, 0};
-    e = bqb::ipm_launch_prepared(d, place, bytes, (cudaStream_t)stream);
+    e = bqb::ipm_launch_prepared(d, optin, (cudaStream_t)stream);
     if (e != cudaSuccess) {
         bqb::set_error("bqb_ipm_noalloc", cudaGetErrorString(e));
         return 2;

@@ -34,6 +34,7 @@
 #include <math.h>
 
 #include "bundle_body.cuh"
+#include "cta_linalg.cuh"
 #include "cuts.cuh"
 #include "ipm_reg_body.cuh"
 #include "kgon_sa.cuh"
@@ -46,6 +47,7 @@ namespace bqb {
 namespace {
 
 constexpr int NKT = IPM_THREADS;
+constexpr size_t NK_STATIC_SMEM = 6144;   // at least the kernel's static shared memory
 constexpr double NK_BIG = 1e9;          // BIG_NUMBER, src/biqbin.h:35
 constexpr int NK_RAND_MAX = 2147483647;
 constexpr int NK_MAX_GW_ROUNDS = 1000;  // rounds of one heuristic call (each improvement needs a larger cut value)
@@ -400,23 +402,18 @@ __device__ __noinline__ void nk_subproblem(const FusedCfg& c, Nk& k)
 // IPM (the engine's kernel body)
 // ---------------------------------------------------------------------------
 // Separate (not inlined) so the IPM body keeps the whole register budget.
-// (The IPM body takes the shared memory as a generic pointer: measured
-// faster here than naming nk_smem inside.)
-__device__ __noinline__ void nk_ipm_call(IpmDesc d, double* smem, int zi, double* stats)
+__device__ __noinline__ void nk_ipm_call(IpmDesc d, int smem_doubles, double* stats)
 {
-    ipm_body_reg(d, smem, zi, stats);
+    ipm_body_reg(d, smem_doubles, stats);
 }
 
 __device__ bool nk_ipm(const FusedCfg& c, Nk& k, const double* Lsrc, double* Xdst, const int* xslot)
 {
     const int n = k.n;
-    const size_t fixed = ipm_reg_fixed_smem_doubles(n) * sizeof(double);
-    const size_t mat = (size_t)n * n * sizeof(double);
-    const int zi = fixed + 2 * mat <= c.smem_bytes ? 1 : 0;
     IpmDesc d{Lsrc, Xdst, k.ws, k.out, xslot, n, 0};
     {
         NkTimer tm(c.prof, NKP_IPM);
-        nk_ipm_call(d, nk_smem, zi, c.ipm_stats);
+        nk_ipm_call(d, (int)(c.smem_bytes / sizeof(double)), c.ipm_stats);
     }
     __syncthreads();
     if ((int)k.out[2] != IPM_OK) {
@@ -1584,9 +1581,9 @@ size_t nk_smem_bytes(int N0, int T, int bcap, size_t smem_optin)
     const size_t n = (size_t)N0, nn = n * n, nv = (n + 1) & ~(size_t)1;
     size_t need = 0;
     auto up = [&](size_t b) { need = b > need ? b : need; };
-    // IPM: fixed part + F, and Zi too when both fit (as the engine places them)
-    const size_t ipm1 = (ipm_reg_fixed_smem_doubles(N0) + nn) * sizeof(double);
-    up(ipm1 + nn * sizeof(double) <= smem_optin ? ipm1 + nn * sizeof(double) : ipm1);
+    // IPM: as many of its matrices as fit beside the kernel's static shared
+    // memory
+    up(ipm_st_smem_doubles_upto(N0, (smem_optin - NK_STATIC_SMEM) / sizeof(double)) * sizeof(double));
     // lambda_eta
     up(le_smem_bytes(bcap < QP_SMEM_K ? bcap : QP_SMEM_K) + 3 * (size_t)bcap * sizeof(double));
     // heuristic: Z, column buffer, d, 16 warps x (Lx, x)
@@ -1609,7 +1606,7 @@ size_t nk_layout(FusedCfg& c)
     sz[NK_L] = nn * 8;
     sz[NK_L0] = nn * 8;
     sz[NK_X] = nn * 8;
-    sz[NK_IPMWS] = 3 * nn * 8;
+    sz[NK_IPMWS] = ipm_st_ws_doubles(c.N0) * 8;
     sz[NK_OUT] = 8 * 8;
     sz[NK_XB] = (size_t)c.bcap * nn * 8;
     sz[NK_G] = M * c.bcap * 8;

@@ -52,82 +52,9 @@ __device__ __forceinline__ void rm_store(const RegMat& M, double* A, int n)
     }
 }
 
-// Store only the lower triangle (r >= c).
-__device__ __forceinline__ void rm_store_lower(const RegMat& M, double* A, int n)
-{
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        const int c = rm_col(b);
-        if (c >= n) continue;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int r = rm_row(a);
-            if (r < n && r >= c) A[r + (size_t)c * n] = M.m[a][b];
-        }
-    }
-}
-
 // Pivot-column buffers of RM_BUF doubles: the column (zeros where the step
 // must not act) and the pivot at RM_NMAX.
 constexpr int RM_BUF = RM_NMAX + 2;
-
-// Owner warp of column k: publish rows r > k of column k (zeros elsewhere,
-// so the update needs no index tests) and the pivot.
-__device__ __forceinline__ void rm_publish_tail(const RegMat& M, int k, double* buf)
-{
-    if ((threadIdx.x >> 5) != (k & 15)) return;
-    const int kb = k >> 4;
-    double v[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) v[a] = 0.0;
-#pragma unroll
-    for (int b = 0; b < 8; ++b)
-        if (b == kb)
-#pragma unroll
-            for (int a = 0; a < 4; ++a) v[a] = M.m[a][b];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int r = rm_row(a);
-        buf[r] = r > k ? v[a] : 0.0;
-        if (r == k) buf[RM_NMAX] = v[a];
-    }
-}
-
-// Is the symmetric matrix in M (lower triangle read) positive definite?
-// The pivots of the symmetric elimination, as a Cholesky factorisation
-// meets them: step k reads the published tail of column k (rows r > k;
-// zeros for r <= k, and the padding rows hold zeros, so the update needs no
-// index tests) and the pivot a_kk, and every thread applies
-// A_ij -= (a_ik / a_kk) a_jk to its 32 entries (a no-op where either factor
-// is zero).  Only the pivots are needed, so the factor itself is not formed
-// (the owner warp has no extra work on the step's critical path).  Returns
-// false, uniformly, at the first non-positive pivot; M is overwritten.
-// col2: 2 * RM_BUF doubles of shared memory.
-__device__ __forceinline__ bool rm_posdef(RegMat& M, int n, double* col2)
-{
-    rm_publish_tail(M, 0, col2);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, tc = threadIdx.x >> 5;
-    for (int k = 0; k < n; ++k) {
-        const double* col = col2 + (k & 1) * RM_BUF;
-        const double d = col[RM_NMAX];
-        if (!(d > 0.0)) return false;
-        const double rs = rsqrt(d);   // 1/sqrt(d); the pivots stay well conditioned here
-        const double inv = rs * rs;
-        double cr[4], cc[8];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) cr[a] = col[lane + 32 * a] * inv;
-#pragma unroll
-        for (int b = 0; b < 8; ++b) cc[b] = col[tc + 16 * b];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 8; ++b) M.m[a][b] = fma(-cr[a], cc[b], M.m[a][b]);
-        if (k + 1 < n) rm_publish_tail(M, k + 1, col2 + ((k + 1) & 1) * RM_BUF);
-        __syncthreads();
-    }
-    return true;
-}
 
 // Owner warp of column k: publish the whole column (rows beyond n hold 0).
 __device__ __forceinline__ void rm_publish_full(const RegMat& M, int k, double* buf)
