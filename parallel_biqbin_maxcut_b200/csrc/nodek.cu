@@ -39,7 +39,7 @@
 #include "ipm_reg_body.cuh"
 #include "kgon_sa.cuh"
 #include "nodek.h"
-#include "trisep.cuh"
+#include "trisep_replay.cuh"
 #include "warm_body.cuh"
 
 namespace bqb {
@@ -48,6 +48,7 @@ namespace {
 
 constexpr int NKT = IPM_THREADS;
 constexpr size_t NK_STATIC_SMEM = 6144;   // at least the kernel's static shared memory
+static_assert(NKT == TR_THREADS, "the separation's replay is a CTA of TR_THREADS threads");
 constexpr double NK_BIG = 1e9;          // BIG_NUMBER, src/biqbin.h:35
 constexpr int NK_RAND_MAX = 2147483647;
 constexpr int NK_MAX_GW_ROUNDS = 1000;  // rounds of one heuristic call (each improvement needs a larger cut value)
@@ -642,29 +643,6 @@ __device__ __forceinline__ void nk_pair_decode(long long p, int* i, int* j)
     *j = (int)(p - (long long)ii * (ii - 1) / 2);
 }
 
-__device__ __forceinline__ bool nk_heap_less(const double* hv, const int* hs, int a, int b)
-{
-    return hv[a] < hv[b] || (hv[a] == hv[b] && hs[a] < hs[b]);
-}
-
-__device__ void nk_heap_down(double* hv, int* hs, int T, int i)
-{
-    while (true) {
-        const int l = 2 * i + 1, r = l + 1;
-        int m = i;
-        if (l < T && nk_heap_less(hv, hs, l, m)) m = l;
-        if (r < T && nk_heap_less(hv, hs, r, m)) m = r;
-        if (m == i) return;
-        const double tv = hv[i];
-        hv[i] = hv[m];
-        hv[m] = tv;
-        const int ts = hs[i];
-        hs[i] = hs[m];
-        hs[m] = ts;
-        i = m;
-    }
-}
-
 // Returns the maximum violation; list in k.tslist, its size in *size.
 __device__ __noinline__ double nk_trisep(const FusedCfg& c, Nk& k, const double* X, int* size)
 {
@@ -739,48 +717,14 @@ __device__ __noinline__ double nk_trisep(const FusedCfg& c, Nk& k, const double*
     }
     const long long V = nk_si[4];
     __syncthreads();
-    // streaming top-T replay by warp 0 (trisep.cu tri_replay_kernel)
-    double* hv = smem;   // XT is dead
-    int* hs = (int*)(hv + (T > 0 ? T : 1));
-    if (warp == 0) {
-        if (T <= 0) {
-            if (lane == 0) nk_si[6] = 0;
-        } else if (V <= T) {
-            for (long long q = lane; q < V; q += 32) k.tslist[q] = k.tscand[q];
-            if (lane == 0) nk_si[6] = (int)V;
-        } else {
-            for (int q = lane; q < T; q += 32) {
-                const TriCand cd = k.tscand[q];
-                k.tslist[q] = cd;
-                hv[q] = cd.value;
-                hs[q] = q;
-            }
-            __syncwarp();
-            if (lane == 0)
-                for (int q = T / 2 - 1; q >= 0; --q) nk_heap_down(hv, hs, T, q);
-            __syncwarp();
-            for (long long base = T; base < V; base += 32) {
-                const long long idx = base + lane;
-                const double v = idx < V ? k.tscand[idx].value : -INFINITY;
-                double th = hv[0];
-                unsigned mask = __ballot_sync(0xffffffffu, v > th);
-                while (mask) {
-                    const int l = __ffs(mask) - 1;
-                    const double vl = __shfl_sync(0xffffffffu, v, l);
-                    __syncwarp();
-                    if (lane == 0) {
-                        const int sl = hs[0];
-                        k.tslist[sl] = k.tscand[base + l];
-                        hv[0] = vl;
-                        nk_heap_down(hv, hs, T, 0);
-                    }
-                    __syncwarp();
-                    th = hv[0];
-                    mask = __ballot_sync(0xffffffffu, lane > l && v > th);
-                }
-            }
-            if (lane == 0) nk_si[6] = T;
-        }
+    // streaming top-T replay (XT is dead)
+    if (T <= 0 || V <= T) {
+        for (long long q = tid; T > 0 && q < V; q += nt) k.tslist[q] = k.tscand[q];
+        if (tid == 0) nk_si[6] = T > 0 ? (int)V : 0;
+    } else {
+        if (tid == 0) nk_si[6] = T;
+        if (!(tr_smem_bytes(T) <= c.smem_bytes && tr_replay_cta(k.tscand, V, T, k.tslist, smem)) && warp == 0)
+            tr_replay_warp(k.tscand, V, T, k.tslist, smem);
     }
     __syncthreads();
     *size = nk_si[6];
@@ -1590,7 +1534,9 @@ size_t nk_smem_bytes(int N0, int T, int bcap, size_t smem_optin)
     up((nn + 2 * nv + (size_t)(NKT / 32) * 2 * nv) * sizeof(double));
     // triangle separation: X^T, then the heap
     up(nn * sizeof(double));
-    up((size_t)(T > 0 ? T : 1) * (sizeof(double) + sizeof(int)) + 16);
+    const size_t Tr = T > 0 ? T : 1;
+    const size_t whole = tr_smem_bytes((int)Tr);
+    up(whole <= smem_optin - NK_STATIC_SMEM ? whole : Tr * (sizeof(double) + sizeof(int)) + 16);
     // annealing chains: X, temperature, 256 permutations
     up((nn + 2) * sizeof(double) + n * 256 * sizeof(unsigned short));
     return (need + 255) & ~(size_t)255;
