@@ -20,6 +20,9 @@
 // condition number of 1e11 at the last iteration, and C D^{-1} C^T then
 // turned a pivot of the positive definite M negative.
 //
+// A sweep holds the lower tiles only (row-major, 32 x 32; the diagonal tiles
+// whole); the final phase of a full sweep writes both triangles.
+//
 // One grid barrier per panel: every CTA factors the 32 x 32 panel block
 // itself (the same arithmetic in every CTA, hence the same decision), and
 // the owner of a 32 x 32 tile of A computes the V rows it needs itself.  The
@@ -27,13 +30,23 @@
 // with the other CTAs' reads of the panel columns, so they are deferred:
 // panel K leaves W_K and D^{-1}_K in side buffers, and in the next phase the
 // owner of each tile in row or column block K writes them before its own
-// update (readers of those entries take them from the side buffers).
+// update, while readers of the panel columns take them from the buffers.
 //
-// Products with F replace the Cholesky solves, each followed by one step of
+// What bounds a phase is its latency (n = 343, cycles): the barrier 3000, one
+// round trip to L2 1600 (the panel block, and the CTA's first tile and its panel
+// columns, are loaded together, from addresses worked out before the barrier),
+// the panel block's chain of 32 pivots on one warp 6000, a tile 4000.  A call at
+// n = 343 takes 3.8 ms, at n = 150 1.7 ms (with rank-1 panel factors by rows,
+// tiles on the vector pipe and every tile of both triangles 10.2 and 4.1).  All
+// products go through the FP64 tensor instruction as X Y^T of 8 x 8 tiles in
+// its accumulators' layout (a lane's pair of columns is also its operand of
+// the two k = 4 steps); V comes from L by tile columns, each solve with a
+// diagonal tile's inverse and one correction.
+//
+// Each solve with M is the product with F = inv(M) followed by one step of
 // iterative refinement with M = Zi .* X (x <- x + F (b - M x)).
 //
-// The grid barrier is a counter and a generation word in global memory;
-// every wait is bounded (2 s), after which the barrier sets an error word,
+// The grid barrier is a growing counter in global memory; every wait is bounded (2 s), after which the barrier sets an error word,
 // no CTA waits any more, every loop ends, and the call reports status
 // IPM_SYNC (a fatal error on the host).
 #include <math.h>
@@ -45,6 +58,7 @@
 #include "bqb_common.cuh"
 #include "internal.h"
 #include "ipm.cuh"
+#include "sym_tiles.cuh"
 
 namespace bqb {
 
@@ -55,8 +69,10 @@ namespace {
 constexpr int CB = 32;          // panel and tile width
 constexpr int CT = 256;         // threads per CTA
 constexpr int CW = CT / 32;     // warps per CTA
-constexpr int LDS = CB + 1;     // padded shared-memory row
-static_assert(CT == CW * 32 && CB == 32 && 4 * CW == CB, "a CTA's threads cover a tile as 32 rows x 8 columns, 4 times");
+// Shared-memory rows of 40 doubles: the pairs of a fragment (eight rows, four
+// pairs each) then meet every bank once.
+constexpr int LD = CB + 8;
+static_assert(CT == CW * 32 && CB == 32 && CW == 8, "a CTA's eight warps hold two of a tile's 16 fragments each");
 constexpr unsigned long long BAR_TIMEOUT_NS = 2000000000ull;
 
 struct CoopArgs {
@@ -69,7 +85,7 @@ struct CoopArgs {
     double *Wb, *Db;                     // 2 x (n x CB), 2 x (CB x CB)
     double *y, *zd, *dy, *dy1, *dy2, *r, *t;
     double* part;        // gridDim.x x 4 partial sums
-    unsigned* bar;       // [0] arrivals, [1] generation, [2] error
+    unsigned* bar;       // [0] arrivals, [2] error
     unsigned long long* prof;   // (may be null) CTA 0's nanoseconds per part, COOP_PROF_* slots
     double* yout;        // (may be null) y of the last iterate
     int n;
@@ -92,26 +108,50 @@ enum CoopProf : int {
 // factor in shared memory).
 constexpr int NTRIAL = 4;
 
-// One panel's factorisation.
-struct PanelF {
-    double Lc[CB][CB];       // the panel's factor by columns (row Q = column Q)
-    double Lr[CB][CB + 2];   // the panel's factor by rows (rows 16-byte aligned)
-    double D[CB][LDS];       // the panel block
-    double Li[CB][LDS];      // inverse of the factor (lower)
-    double R[CB];            // reciprocals of the factor's diagonal
-};
+using Block = double[CB][LD];
 
+// Shared memory: a trial's panel factor (L, the inverses Y of its diagonal tiles,
+// G = L^{-T}), the tile step's V_I, V_J in two sets; the products' two sets of four operands and their
+// transposes' scratch.
 struct Smem {
-    PanelF pf[NTRIAL];
-    double A1[CB][LDS];   // C_I, or a GEMM operand tile
-    double A2[CB][LDS];   // C_J, or a GEMM operand tile
-    double V1[CB][LDS];   // V_I, or a GEMM operand tile
-    double V2[CB][LDS];   // V_J, or a GEMM operand tile
+    Block b[3 * NTRIAL + 4];
     double red[CW * 4];
     double tot[4];
+    // what the sweeps use of the call's arguments: an acquire empties L1, and
+    // with it whatever a function keeps in local memory
+    double* A[NTRIAL];
+    double *Wb, *Db;
+    unsigned* bar;
+    unsigned epoch;   // grid barriers passed
     int ok;
     int pd[NTRIAL];
+    __device__ Block& Y(int t) { return b[2 * t]; }
+    __device__ Block& G(int t) { return b[2 * t + 1]; }
+    __device__ Block& L(int t) { return b[2 * NTRIAL + t]; }
+    __device__ Block& V(int set, int side) { return b[3 * NTRIAL + 2 * set + side]; }
 };
+
+// This lane's fragment of 8 x 8 tile (I, J) of a block: row lane / 4, columns
+// 2 (lane % 4) and + 1.
+__device__ __forceinline__ double2 frag(const Block& m, int I, int J)
+{
+    const int lane = threadIdx.x & 31;
+    return *reinterpret_cast<const double2*>(&m[8 * I + (lane >> 2)][8 * J + 2 * (lane & 3)]);
+}
+__device__ __forceinline__ void put(Block& m, int I, int J, const double2& v)
+{
+    const int lane = threadIdx.x & 31;
+    *reinterpret_cast<double2*>(&m[8 * I + (lane >> 2)][8 * J + 2 * (lane & 3)]) = v;
+}
+// ... and the transposed tile at (J, I).
+__device__ __forceinline__ void put_t(Block& m, int I, int J, const double2& v)
+{
+    const int lane = threadIdx.x & 31, r = 8 * J + 2 * (lane & 3), c = 8 * I + (lane >> 2);
+    m[r][c] = v.x;
+    m[r + 1][c] = v.y;
+}
+__device__ __forceinline__ void mma(double2& c, const double2& a, const double2& b) { st_mma(c.x, c.y, a, b); }
+__device__ __forceinline__ double2 neg(const double2& a) { return make_double2(-a.x, -a.y); }
 
 __device__ __forceinline__ unsigned long long global_ns()
 {
@@ -120,40 +160,39 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
-// Grid barrier with a bounded wait.  Returns false once any CTA has given up
-// (then nothing waits any more).  The fences around the arrival make every
-// write before the barrier visible to every read after it.
+// Grid barrier with a bounded wait: one counter that only grows, a CTA
+// waiting until all have added to it as often as itself.  Returns false once
+// any CTA has given up (then nothing waits any more).  The fences around the
+// arrival make every write before the barrier visible to every read after it.
 __device__ bool grid_sync(unsigned* bar, Smem& sm, unsigned long long* prof = nullptr)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned long long tb = prof && blockIdx.x == 0 ? global_ns() : 0ull;
-        volatile unsigned* vb = bar;
-        int ok = vb[2] == 0u;
-        if (ok) {
-            const unsigned gen = vb[1];
-            __threadfence();
-            if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-                atomicExch(bar, 0u);
-                __threadfence();
-                atomicAdd(bar + 1, 1u);
-            } else {
-                const unsigned long long t0 = global_ns();
-                while (vb[1] == gen) {
-                    if (vb[2] != 0u) {
-                        ok = 0;
-                        break;
-                    }
-                    if (global_ns() - t0 > BAR_TIMEOUT_NS) {
-                        atomicExch(bar + 2, 1u);
-                        ok = 0;
-                        break;
-                    }
-                    __nanosleep(32);
+        const unsigned target = (sm.epoch += 1) * gridDim.x;
+        int ok = 1;
+        __threadfence();
+        asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        unsigned long long t0 = 0ull;
+        for (unsigned spin = 1;; ++spin) {
+            unsigned v;
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if ((spin & 255u) == 0u) {
+                const unsigned long long now = global_ns();
+                if (!t0) t0 = now;
+                if (*(volatile unsigned*)(bar + 2) != 0u) {
+                    ok = 0;
+                    break;
+                }
+                if (now - t0 > BAR_TIMEOUT_NS) {
+                    atomicExch(bar + 2, 1u);
+                    ok = 0;
+                    break;
                 }
             }
-            __threadfence();
         }
+        __threadfence();
         sm.ok = ok;
         if (prof && blockIdx.x == 0) {
             prof[COOP_PROF_BARRIER] += global_ns() - tb;
@@ -165,10 +204,15 @@ __device__ bool grid_sync(unsigned* bar, Smem& sm, unsigned long long* prof = nu
 }
 
 // The sums over all entries (the starting point's, the step's) are taken
-// over a fixed partition into VCTA parts, one block of CT threads each with
-// the entries of a CTA of a VCTA-CTA grid; a CTA of a smaller grid takes
+// over a fixed partition into as many parts as give a thread four entries (at
+// most VCTA), a block of CT threads each; a CTA of a smaller grid takes
 // several parts in turn.  The totals are then the same bits for any grid.
 constexpr int VCTA = 148;
+__device__ __forceinline__ int sum_parts(int n)
+{
+    const long long p = ((long long)n * n + 4 * CT - 1) / (4 * CT);
+    return p < VCTA ? (int)p : VCTA;
+}
 
 // Block-reduce four partial sums into part[v * 4 + k] (the CTA's part v).
 __device__ void block_partials(double a, double b, double c, double d, Smem& sm, double* part, int v)
@@ -193,488 +237,663 @@ __device__ void block_partials(double a, double b, double c, double d, Smem& sm,
     __syncthreads();   // sm.red is reused by the CTA's next part
 }
 
-// The totals of the partial sums (after a barrier), in part order: the same
-// value in every CTA.
-__device__ void grid_totals(const double* part, Smem& sm)
+// The totals of the partial sums (after a barrier), a warp each, in a fixed
+// order: the same value in every CTA.
+__device__ void grid_totals(const double* part, int parts, Smem& sm)
 {
-    if (threadIdx.x < 4) {
-        double s = 0.0;
-        for (int g = 0; g < VCTA; ++g) s += part[g * 4 + threadIdx.x];
-        sm.tot[threadIdx.x] = s;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    static_assert(VCTA <= 5 * 32, "a lane's five parts");
+    if (w < 4) {
+        double v[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) v[q] = lane + 32 * q < parts ? __ldcg(part + (lane + 32 * q) * 4 + w) : 0.0;
+        const double s = warp_sum((((v[0] + v[1]) + v[2]) + v[3]) + v[4]);
+        if (lane == 0) sm.tot[w] = s;
     }
     __syncthreads();
 }
 
 // ---- the panel sweep ---------------------------------------------------------
 
-// Step Q of the register Cholesky of a 32 x 32 block held by one warp
-// (lane p holds row p in s[]): column Q of the factor, then the rank-1
-// update of the rows below.  The column goes to the warp through shared
-// memory (one store per lane, then broadcast reads of two entries at a
-// time), which costs fewer issue slots than a shuffle per entry.
-// Instantiated for every Q so that every index into s[] is a constant and
-// s[] stays in registers.  No early exit: after a non-positive pivot (the
-// same d in every lane) the steps go on with a unit pivot and the caller
-// discards the result.  Lane Q keeps the pivot's reciprocal square root, the
-// reciprocal of its diagonal entry of the factor.
-template <int Q>
-__device__ __forceinline__ void chol_step(double (&s)[CB], int p, int& pd, double& rdiag, double (*Lc)[CB])
+// Named barrier by which trial t's chain warp hands tile columns up to K of
+// the factor to its helper (K = 1, 2, 3; 64 threads).
+__device__ __forceinline__ int hand_over(int t, int K) { return 3 * t + K; }
+static_assert(3 * NTRIAL < 16, "named barriers");
+
+// a y^T (y = L^{-1}: x with x L^T = a).
+__device__ __forceinline__ double2 solve_t(const double2& a, const double2& y)
 {
-    if constexpr (Q < CB) {
-        double d = __shfl_sync(0xffffffffu, s[Q], Q);
-        if (!(d > 0.0)) {
-            pd = 0;
-            d = 1.0;
-        }
-        const double rs = rsqrt(d);
-        const double l = d * rs;
-        const double lpq = p == Q ? l : s[Q] * rs;
-        if (p == Q) rdiag = rs;
-        s[Q] = lpq;
-        Lc[Q][p] = lpq;
-        __syncwarp();
-        constexpr int r0 = (Q + 1) & ~1;
-#pragma unroll
-        for (int r = r0; r < CB; r += 2) {
-            const double2 v = *reinterpret_cast<const double2*>(&Lc[Q][r]);
-            if (r > Q && r <= p) s[r] = fma(-lpq, v.x, s[r]);
-            if (r + 1 <= p) s[r + 1] = fma(-lpq, v.y, s[r + 1]);
-        }
-        chol_step<Q + 1>(s, p, pd, rdiag, Lc);
-    }
+    double2 x = make_double2(0.0, 0.0);
+    mma(x, a, y);
+    return x;
 }
 
-// Step I of the inverse of the lower factor for the calling lane's column t:
-// li[I] = (delta_It - sum_{k < I} Lr[I][k] li[k]) / Lr[I][I] (zero above the
-// diagonal, where every term is zero).  Instantiated for every I so that li[]
-// stays in registers; the factor's entries are shared-memory broadcasts read
-// two at a time that do not depend on the chain.  The sum runs in four
-// interleaved partial sums, so the dependent chain per step is a quarter as
-// long.
-template <int I>
-__device__ __forceinline__ void linv_step(double (&li)[CB], const PanelF& sm, int t)
+// The panel block D = A[K, K] (b x b, padded to 32 x 32 with the identity), its
+// lower tiles, by one warp; a: this lane's first pair.
+struct PanelTiles {
+    double2 d[4][4];
+};
+__device__ __forceinline__ void panel_load(const double* a, unsigned n, int b, PanelTiles& f)
 {
-    if constexpr (I < CB) {
-        double a0 = I == t ? 1.0 : 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+    const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
 #pragma unroll
-        for (int k = 0; k + 3 < I; k += 4) {
-            const double2 u = *reinterpret_cast<const double2*>(&sm.Lr[I][k]);
-            const double2 w = *reinterpret_cast<const double2*>(&sm.Lr[I][k + 2]);
-            a0 = fma(-u.x, li[k], a0);
-            a1 = fma(-u.y, li[k + 1], a1);
-            a2 = fma(-w.x, li[k + 2], a2);
-            a3 = fma(-w.y, li[k + 3], a3);
-        }
+    for (int I = 0; I < 4; ++I)
 #pragma unroll
-        for (int k = I & ~3; k < I; ++k) a0 = fma(-sm.Lr[I][k], li[k], a0);
-        li[I] = ((a0 + a1) + (a2 + a3)) * sm.R[I];
-        linv_step<I + 1>(li, sm, t);
-    }
-}
-
-// The panel block D = A[K, K] (b x b, padded to 32 x 32 with the identity)
-// into f.D; every thread of the CTA takes part (no barrier).
-__device__ __forceinline__ void panel_load(const double* A, int n, int k0, int b, PanelF& f)
-{
-    for (int e = threadIdx.x; e < CB * CB; e += CT) {
-        const int p = e % CB, q = e / CB;
-        f.D[p][q] = p < b && q < b ? A[(k0 + p) + (size_t)(k0 + q) * n] : (p == q ? 1.0 : 0.0);
-    }
-}
-
-// One warp: the Cholesky factor Ld of f.D and Li = Ld^{-1} in f (lane p
-// holds row p in registers), then lane t forms column t of Li by forward
-// substitution.  *pd_out = 0 on a non-positive pivot (then f is partial).
-__device__ void panel_chol(PanelF& sm, int* pd_out)
-{
-    {
-        const int p = threadIdx.x & 31;
-        double s[CB];
-#pragma unroll
-        for (int r = 0; r < CB; ++r) s[r] = sm.D[p][r];
-        int pd = 1;
-        double rdiag = 1.0;
-        chol_step<0>(s, p, pd, rdiag, sm.Lc);
-        if (p == 0) *pd_out = pd;
-        if (pd) {
-#pragma unroll
-            for (int r = 0; r < CB; r += 2)
-                *reinterpret_cast<double2*>(&sm.Lr[p][r]) = make_double2(r <= p ? s[r] : 0.0, r + 1 <= p ? s[r + 1] : 0.0);
-            sm.R[p] = rdiag;
-        }
-        __syncwarp();
-        if (pd) {
-            double li[CB];
-            linv_step<0>(li, sm, p);
-#pragma unroll
-            for (int i = 0; i < CB; ++i) sm.Li[i][p] = li[i];
-        }
-    }
-}
-
-// Every CTA: the Cholesky factor Ld of D = A[K, K] (b x b) and Li = Ld^{-1}
-// in sm.pf[0] (warp 0 factors).  Returns false (in every thread) on a
-// non-positive pivot.
-__device__ bool panel_factor(const double* A, int n, int k0, int b, Smem& sm, unsigned long long* load_ns)
-{
-    const unsigned long long t0 = load_ns ? global_ns() : 0ull;
-    panel_load(A, n, k0, b, sm.pf[0]);
-    __syncthreads();
-    if (load_ns) *load_ns += global_ns() - t0;
-    if (threadIdx.x < 32) panel_chol(sm.pf[0], &sm.pd[0]);
-    __syncthreads();
-    return sm.pd[0] != 0;
-}
-
-// C rows of tile block I (32 x b): the panel columns of A for rows I, or, for
-// the row block of the previous panel (whose entries still wait for their
-// fix), W_{K-1} transposed.  Then V = C Ld^{-T}: V(r, q) = sum_{p <= q}
-// C(r, p) Li(q, p).  Not inlined: its registers are then allocated apart
-// from the panel factorisation's, and the kernel needs no spill slots.
-__device__ __noinline__ void load_v(const double* A, int n, int I, int k0, int b, const double* Wprev, bool from_w,
-                       double (*Cs)[LDS], double (*Vs)[LDS], const PanelF& f)
-{
-    const int i0 = I * CB;
-    for (int e = threadIdx.x; e < CB * CB; e += CT) {
-        const int r = e % CB, p = e / CB;
-        const int i = i0 + r;
-        double v = 0.0;
-        if (i < n && p < b) v = from_w ? Wprev[(k0 + p) + (size_t)r * n] : A[i + (size_t)(k0 + p) * n];
-        Cs[r][p] = v;
-    }
-    __syncthreads();
-    // thread (r, c0) forms V(r, c0 + 8 j), j = 0..3, reading C(r, p) once for
-    // all four; Li(q, p) = 0 for p > q, so running p to the largest q adds
-    // exact zeros to the smaller ones
-    {
-        const int r = threadIdx.x % CB, c0 = threadIdx.x / CB;
-        double v[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int p = 0; p <= c0 + 3 * CW; ++p) {
-            const double cp = Cs[r][p];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = fma(cp, f.Li[c0 + CW * j][p], v[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) Vs[r][c0 + CW * j] = c0 + CW * j < b ? v[j] : 0.0;
-    }
-    __syncthreads();
-}
-
-// Phase K of the sweep for tile (I, J).  FULL: the pending fix of panel
-// K - 1 (tiles in its row or column block), the update (I, J != K), W_K of
-// row block I (diagonal tiles) and D^{-1}_K (tile (K, K)).  Trailing only:
-// the update.
-template <bool FULL>
-__device__ void tile_step(double* A, int n, int K, int k0, int b, int I, int J, const double* Wprev,
-                          const double* Dprev, double* Wcur, double* Dcur, Smem& sm, const PanelF& f)
-{
-    const bool fixI = FULL && K > 0 && I == K - 1;
-    const bool fixJ = FULL && K > 0 && J == K - 1;
-    const bool upd = I != K && J != K;
-    if (!upd && !fixI && !fixJ && !(FULL && I == K && J == K)) return;
-    if (upd) {
-        load_v(A, n, I, k0, b, Wprev, fixI, sm.A1, sm.V1, f);
-        if (J != I) load_v(A, n, J, k0, b, Wprev, fixJ, sm.A2, sm.V2, f);
-    }
-    double (*VJ)[LDS] = J != I ? sm.V2 : sm.V1;
-    const int i0 = I * CB, j0 = J * CB, kp0 = (K - 1) * CB;
-    // thread (r, c0) owns the entries (r, c0 + 8 j), j = 0..3, of the tile
-    // and reads V1(r, q) once for all four
-    const int r = threadIdx.x % CB, c0 = threadIdx.x / CB;
-    if (upd || fixI || fixJ) {
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        if (upd)
-            for (int q = 0; q < b; ++q) {
-                const double a = sm.V1[r][q];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) acc[jj] = fma(a, VJ[c0 + CW * jj][q], acc[jj]);
+        for (int J = 0; J <= I; ++J) {
+            const double* x = a + 8 * I * n + 8 * J;
+            if (b == CB) {
+                f.d[I][J] = make_double2(__ldcg(x), __ldcg(x + 1));
+            } else {
+                const int p = 8 * I + r, q = 8 * J + 2 * c;
+                f.d[I][J].x = p < b && q < b ? __ldcg(x) : (p == q ? 1.0 : 0.0);
+                f.d[I][J].y = p < b && q + 1 < b ? __ldcg(x + 1) : (p == q + 1 ? 1.0 : 0.0);
             }
+        }
+}
+
+// Its Cholesky factor L (tiles below the diagonal, in sm.L(t)) and the inverses
+// Y of L's diagonal tiles (sm.Y(t)), as a factorisation of 4 x 4 tiles: a tile's
+// eight pivots are st_chol_inv's chain (1000 cycles), the column below them and
+// the trailing tiles are tensor products in registers.  5100 cycles; the 32
+// steps of a rank-1 update by rows, and the substitution for the inverse after
+// them, took 20000.  sm.pd[t] = 0 on a non-positive pivot (then the results are
+// garbage).  helped: panel_help follows on another warp.
+__device__ __forceinline__ void panel_chain(PanelTiles& f, int t, bool helped, Smem& sm)
+{
+    double2 (&d)[4][4] = f.d;
+    Block& yb = sm.Y(t);
+    Block& lo = sm.L(t);
+    bool pd = true;
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const int c = c0 + CW * jj;
-            const int i = i0 + r, j = j0 + c;
-            if (i >= n || j >= n) continue;
-            double v;
-            if (fixI && fixJ) v = -Dprev[(i - kp0) + (size_t)(j - kp0) * CB];
-            else if (fixJ) v = Wprev[i + (size_t)(j - kp0) * n];
-            else if (fixI) v = Wprev[j + (size_t)(i - kp0) * n];
-            else v = A[i + (size_t)j * n];
-            if (upd) v -= acc[jj];
-            A[i + (size_t)j * n] = v;
+    for (int K = 0; K < 4; ++K) {
+        double2 y;
+        const bool ok = st_chol_inv(d[K][K], y);
+        pd = pd && ok;
+        put(yb, K, K, y);
+#pragma unroll
+        for (int I = K + 1; I < 4; ++I) {
+            d[I][K] = solve_t(d[I][K], y);
+            put(lo, I, K, d[I][K]);
+        }
+        if (K > 0 && helped) st_bar_arrive(hand_over(t, K), 64);
+#pragma unroll
+        for (int I = K + 1; I < 4; ++I)
+#pragma unroll
+            for (int J = K + 1; J <= I; ++J) mma(d[I][J], neg(d[I][K]), d[J][K]);
+    }
+    if ((threadIdx.x & 31) == 0) sm.pd[t] = pd ? 1 : 0;
+}
+
+// The helper, for a full sweep: G = L^{-T} (upper tiles), column K when the
+// chain has tile column K: G_JK = -(sum_{J <= m < K} G_Jm L_Km^T) L_KK^{-T}.
+__device__ __forceinline__ void panel_help(int t, Smem& sm)
+{
+    const Block& yb = sm.Y(t);
+    Block& g = sm.G(t);
+    const Block& lo = sm.L(t);
+    double2 gt[4][4];   // upper tiles
+#pragma unroll
+    for (int K = 0; K < 4; ++K) {
+        if (K > 0) st_bar_sync(hand_over(t, K), 64);
+        if (K == 0) continue;
+#pragma unroll
+        for (int k = K == 1 ? 0 : K; k <= K; ++k) {
+            const double2 y = frag(yb, k, k);
+            put_t(g, k, k, y);
+            __syncwarp();
+            gt[k][k] = frag(g, k, k);
+#pragma unroll
+            for (int J = 0; J < k; ++J) {
+                double2 x = make_double2(0.0, 0.0);
+#pragma unroll
+                for (int m = J; m < k; ++m) mma(x, gt[J][m], frag(lo, k, m));
+                gt[J][k] = solve_t(neg(x), y);
+                put(g, J, k, gt[J][k]);
+            }
         }
     }
-    if (FULL && upd && I == J) {
-        // W_K(i, q) = sum_{p >= q} V(i, p) Li(p, q); Li(p, q) = 0 for p < q,
-        // so starting p at the smallest q adds exact zeros to the others
-        double w[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int p = c0; p < b; ++p) {
-            const double vp = sm.V1[r][p];
+}
+
+// A CTA's tile of a phase, as it comes from memory: its entries (this warp's two
+// fragments: tile row warp / 2, tile columns 2 (warp & 1) and + 1), and of the
+// panel's columns a strip of eight rows (strip warp & 3 of the tile's rows, or
+// from warp 4 on of its columns' rows).
+struct TileLoad {
+    double2 c[4];
+    double2 a[2];
+};
+
+// Which tile of A the phase gives the CTA, and what is to be done with it.
+struct TileJob {
+    double* A;
+    int I, J;
+    bool full;    // a full sweep's tile: also the previous panel's fix, W, D^{-1}
+    int trial;    // whose panel factor
+};
+
+// Where a thread's values of a tile come from, worked out before the grid
+// barrier (the index arithmetic took as long as the round trip to L2).
+struct TileAddr {
+    const double* c;   // the strip's pairs: columns 8 u + 2 (lane % 4) and + 1, cn of them in range, cs apart
+    const double* a;   // the entries: columns 8 e and + 1, an in range, as apart
+    unsigned cs, as;
+    int cn, an;
+};
+
+__device__ __forceinline__ TileAddr tile_addr(const TileJob& q, int n, int K, int k0, int b, const double* Wprev,
+                                              const double* Dprev)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int I = q.I, J = q.J;
+    const bool upd = I != K && J != K;
+    const bool fixI = q.full && K > 0 && I == K - 1, fixJ = q.full && K > 0 && J == K - 1;
+    const unsigned un = n;
+    TileAddr t;
+    {
+        // rows of the lower triangle, columns of it, or the previous panel's W
+        const int B = w >= 4 ? J : I;
+        const bool from_w = w >= 4 ? fixJ : fixI;
+        const unsigned r = 8 * (w & 3) + (lane >> 2), i = B * CB + r, p = 2 * (lane & 3);
+        t.cs = from_w ? CB : B < K ? un : 1u;
+        t.c = from_w ? Wprev + ((k0 + p) * CB + r) : q.A + (B < K ? (k0 + p) * un + i : i * un + k0 + p);
+        t.cn = upd && (int)i < n && (w < 4 || J != I) ? b - (int)p : 0;
+    }
+    {
+        const unsigned i = I * CB + 8 * (w >> 1) + (lane >> 2), j = J * CB + 16 * (w & 1) + 2 * (lane & 3);
+        const unsigned kp0 = (K - 1) * CB;
+        t.as = fixI && !fixJ ? CB : 1u;
+        t.a = fixI && fixJ ? Dprev + ((i - kp0) * CB + (j - kp0))
+              : fixJ       ? Wprev + (i * CB + (j - kp0))
+              : fixI       ? Wprev + (j * CB + (i - kp0))
+                           : q.A + (i * un + j);
+        t.an = (upd || fixI || fixJ) && (int)i < n ? n - (int)j : 0;
+    }
+    return t;
+}
+
+// Issue the loads (of nothing that the phase writes).
+__device__ __forceinline__ void tile_load(const TileAddr& s, TileLoad& t)
+{
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) w[jj] = fma(vp, f.Li[p][c0 + CW * jj], w[jj]);
+    for (int u = 0; u < 4; ++u) {
+        t.c[u].x = 8 * u < s.cn ? __ldcg(s.c + 8 * u * s.cs) : 0.0;
+        t.c[u].y = 8 * u + 1 < s.cn ? __ldcg(s.c + (8 * u + 1) * s.cs) : 0.0;
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        t.a[e].x = 8 * e < s.an ? __ldcg(s.a + 8 * e * s.as) : 0.0;
+        t.a[e].y = 8 * e + 1 < s.an ? __ldcg(s.a + (8 * e + 1) * s.as) : 0.0;
+    }
+}
+
+// The tile's step, from its loads: the pending fix of panel K - 1 (tiles in
+// its row or column block), the update (I, J != K), and for a full sweep W_K
+// of row block I (diagonal tiles) and D^{-1}_K (tile (K, K)).  One barrier,
+// after the V strips (a warp each), and none without an update: the CTA's next
+// update uses the other set, and its barrier is behind this one's reads.
+__device__ __forceinline__ void tile_step(const TileJob& q, int n, int K, TileLoad& t, double* Wcur, double* Dcur,
+                                          int set, Smem& sm)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int I = q.I, J = q.J;
+    const int ta = w >> 1, tb = 2 * (w & 1);
+    const bool upd = I != K && J != K;
+    const bool fixI = q.full && K > 0 && I == K - 1, fixJ = q.full && K > 0 && J == K - 1;
+    const Block& G = sm.G(q.trial);
+    const int i = I * CB + 8 * ta + (lane >> 2);
+    if (fixI && fixJ) {
+        t.a[0] = neg(t.a[0]);
+        t.a[1] = neg(t.a[1]);
+    }
+    if (upd) {
+        // V L^T = C, tile column by tile column
+        if (w < 4 || J != I) {
+            const Block& L = sm.L(q.trial);
+            const Block& Y = sm.Y(q.trial);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                double2 x = t.c[u];
+#pragma unroll
+                for (int p = 0; p < u; ++p) mma(x, neg(t.c[p]), frag(L, u, p));
+                t.c[u] = solve_t(x, frag(Y, u, u));
+                put(sm.V(set, w >> 2), w & 3, u, t.c[u]);
+            }
         }
-        const int i = i0 + r;
+        __syncthreads();
+        const Block& V = sm.V(set, 0);
+        const Block& VJ = sm.V(set, J != I ? 1 : 0);
+        // (summed apart and subtracted once: 32 roundings at A's size a panel
+        // instead of one made the line searches of problems with couplings of
+        // 2e5 fail)
+        double2 x[2] = {};
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const int q = c0 + CW * jj;
-            if (i < n && q < b) Wcur[i + (size_t)q * n] = w[jj];
+        for (int p = 0; p < 4; ++p) {
+            const double2 v = frag(V, ta, p);
+            mma(x[0], v, frag(VJ, tb, p));
+            mma(x[1], v, frag(VJ, tb + 1, p));
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) t.a[e] = make_double2(t.a[e].x - x[e].x, t.a[e].y - x[e].y);
+    }
+    if (upd || fixI || fixJ) {
+        const int j = J * CB + 8 * tb + 2 * (lane & 3);
+        double* o = q.A + ((unsigned)i * (unsigned)n + (unsigned)j);
+        if (i < n) {
+            if (j < n) o[0] = t.a[0].x;
+            if (j + 1 < n) o[1] = t.a[0].y;
+            if (j + 8 < n) o[8] = t.a[1].x;
+            if (j + 9 < n) o[9] = t.a[1].y;
         }
     }
-    if (FULL && I == K && J == K) {
-        // D^{-1}_K = Li^T Li
-        for (int e = threadIdx.x; e < CB * CB; e += CT) {
-            const int p = e % CB, q = e / CB;
-            double acc = 0.0;
-            for (int k = p > q ? p : q; k < b; ++k) acc = fma(f.Li[k][p], f.Li[k][q], acc);
-            Dcur[p + (size_t)q * CB] = acc;
+    if (q.full && upd && I == J) {
+        // W = V Li = V G^T
+        const Block& V = sm.V(set, 0);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            double2 x = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+                if (p >= tb + e) mma(x, frag(V, ta, p), frag(G, tb + e, p));
+            if (i < n) {
+                double* o = Wcur + (size_t)i * CB + 8 * (tb + e) + 2 * (lane & 3);
+                o[0] = x.x;
+                o[1] = x.y;
+            }
         }
     }
-    __syncthreads();
+    if (q.full && I == K && J == K) {
+        // D^{-1} = Li^T Li = G G^T
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            double2 x = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+                if (p >= ta && p >= tb + e) mma(x, frag(G, ta, p), frag(G, tb + e, p));
+            double* o = Dcur + (8 * ta + (lane >> 2)) * CB + 8 * (tb + e) + 2 * (lane & 3);
+            o[0] = x.x;
+            o[1] = x.y;
+        }
+    }
 }
 
 // The final phase of a full sweep: the fix of the last panel's row and
-// column blocks, and A = -A; with Xm, also Mout = Fout = A .* Xm (Xm + ap dXm
-// with dXm).  No barrier.
-__device__ void sweep_final(double* A, const CoopArgs& a, const double* Xm, double* Mout, double* Fout,
-                            const double* dXm, double ap)
+// column blocks, and A = -A, both triangles; with Xm, also Mout = A .* Xm (both
+// triangles) and Fout's lower tiles the same.  No grid barrier.
+__device__ void sweep_final(double* A, const CoopArgs& a, Smem& sm, const double* Xm, double* Mout, double* Fout)
 {
     const int n = a.n;
     const int T = (n + CB - 1) / CB;
-    {
-        const int K = T;
-        const double* Wl = a.Wb + (size_t)((K + 1) & 1) * n * CB;
-        const double* Dl = a.Db + (size_t)((K + 1) & 1) * CB * CB;
-        const int kp0 = (K - 1) * CB;
-        for (int q = blockIdx.x; q < T * T; q += gridDim.x) {
-            const int I = q % T, J = q / T;
-            const bool fixI = I == K - 1, fixJ = J == K - 1;
-            for (int e = threadIdx.x; e < CB * CB; e += CT) {
-                const int i = I * CB + e % CB, j = J * CB + e / CB;
-                if (i >= n || j >= n) continue;
-                double v;
-                if (fixI && fixJ) v = -Dl[(i - kp0) + (size_t)(j - kp0) * CB];
-                else if (fixJ) v = Wl[i + (size_t)(j - kp0) * n];
-                else if (fixI) v = Wl[j + (size_t)(i - kp0) * n];
-                else v = A[i + (size_t)j * n];
-                const size_t ij = i + (size_t)j * n;
-                A[ij] = -v;
-                if (Xm) {
-                    const double xm = dXm ? fma(ap, dXm[ij], Xm[ij]) : Xm[ij];
-                    const double m = -v * xm;
-                    Mout[ij] = m;
-                    Fout[ij] = m;
-                }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const double* Wl = a.Wb + (size_t)((T + 1) & 1) * n * CB;
+    const double* Dl = a.Db + (size_t)((T + 1) & 1) * CB * CB;
+    const int kp0 = (T - 1) * CB;
+    for (int q = blockIdx.x; q < T * (T + 1) / 2; q += gridDim.x) {
+        int I, J;
+        st_decode(q, &I, &J);
+        const bool fixI = I == T - 1, fixJ = J == T - 1;
+        Block& z = sm.V(0, 0);
+        Block& m = sm.V(0, 1);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = w + CW * k;
+            const int i = I * CB + r, j = J * CB + lane;
+            if (i >= n || j >= n) continue;
+            double v;
+            if (fixI && fixJ) v = -__ldcg(Dl + (i - kp0) * CB + (j - kp0));
+            else if (fixI) v = __ldcg(Wl + (size_t)j * CB + (i - kp0));
+            else v = __ldcg(A + (size_t)i * n + j);
+            const size_t ij = (size_t)i * n + j;
+            A[ij] = -v;
+            z[r][lane] = -v;
+            if (Xm) {
+                const double x = -v * Xm[ij];
+                Mout[ij] = x;
+                Fout[ij] = x;
+                m[r][lane] = x;
             }
         }
-    }
-}
-
-// The panel sweep of A (n x n).  FULL: A becomes inv(A); otherwise only the
-// trailing updates run, for the pivots.  With Xm (FULL only), the final
-// phase also writes Mout = Fout = inv(A) .* Xm for its tiles (the next
-// inverse's input), saving a phase; with dXm as well, Xm + ap dXm (rounded
-// as the step's update rounds it) takes the place of Xm.  Returns 1
-// (positive definite), 0 (a non-positive pivot; every CTA returns 0 at the
-// same panel) or -1 (a barrier gave up).
-template <bool FULL>
-__device__ int sweep(double* A, const CoopArgs& a, Smem& sm, const double* Xm = nullptr, double* Mout = nullptr,
-                     double* Fout = nullptr, const double* dXm = nullptr, double ap = 0.0)
-{
-    const int n = a.n;
-    const int T = (n + CB - 1) / CB;
-    for (int K = 0; K < T; ++K) {
-        const int k0 = K * CB, b = n - k0 < CB ? n - k0 : CB;
-        const bool rec = a.prof && blockIdx.x == 0 && threadIdx.x == 0;
-        unsigned long long tp = rec ? global_ns() : 0ull;
-        if (!panel_factor(A, n, k0, b, sm, rec ? a.prof + COOP_PROF_PF_LOAD : nullptr)) return 0;
-        if (rec) {
-            const unsigned long long t = global_ns();
-            a.prof[COOP_PROF_FACTOR] += t - tp;
-            a.prof[COOP_PROF_PHASES] += 1;
-            tp = t;
+        if (I == J) continue;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = w + CW * k;
+            const int i = J * CB + r, j = I * CB + lane;
+            if (i >= n || j >= n) continue;
+            A[(size_t)i * n + j] = z[lane][r];
+            if (Xm) Mout[(size_t)i * n + j] = m[lane][r];
         }
-        if (!FULL && K == T - 1) return 1;
-        const double* Wprev = a.Wb + (size_t)((K + 1) & 1) * n * CB;
-        const double* Dprev = a.Db + (size_t)((K + 1) & 1) * CB * CB;
-        double* Wcur = a.Wb + (size_t)(K & 1) * n * CB;
-        double* Dcur = a.Db + (size_t)(K & 1) * CB * CB;
-        const int t0 = FULL ? 0 : K + 1;
-        const int Tt = T - t0;
-        for (int q = blockIdx.x; q < Tt * Tt; q += gridDim.x)
-            tile_step<FULL>(A, n, K, k0, b, t0 + q % Tt, t0 + q / Tt, Wprev, Dprev, Wcur, Dcur, sm, sm.pf[0]);
-        if (a.prof) __syncthreads();
-        if (rec) a.prof[COOP_PROF_TILES] += global_ns() - tp;
-        if (!grid_sync(a.bar, sm, a.prof)) return -1;
     }
-    if (FULL) {
-        // the last panel's fix, and A = -A
-        sweep_final(A, a, Xm, Mout, Fout, dXm, ap);
-        if (!grid_sync(a.bar, sm, a.prof)) return -1;
-    }
-    return 1;
 }
 
-// Trial sweeps run together: nt matrices, each the trailing sweep (its
-// pivots) or, for at most one, the full sweep (its inverse).  state[t]
-// becomes 1 (positive definite) or -1 (a non-positive pivot); every CTA takes
-// the same decisions.
+// The panel sweep of A (n x n, lower tiles).  FULL: A becomes inv(A) (both
+// triangles); otherwise only the trailing updates run, for the pivots.  With
+// Xm (FULL only), the final phase also writes Mout = Fout = inv(A) .* Xm (the
+// next inverse's input), saving a phase.  Sweeps run together: nt matrices,
+// at most one of them full.  state[t] becomes 1 (positive definite) or -1 (a
+// non-positive pivot); every CTA takes the same decisions.
 struct TrialSet {
     double* A[NTRIAL];
     int full[NTRIAL];
     int state[NTRIAL];
     int nt;
+    const double* Xm = nullptr;   // (of the full one)
+    double *Mout = nullptr, *Fout = nullptr;
 };
 
 // In each phase every running trial's panel block is factored by its own
-// warp (warp t for trial t) and the tiles of all running trials are spread
-// over the CTAs; a trial drops out at its first non-positive pivot, a
+// warp (warp t for trial t) and the lower tiles of all running trials are
+// spread over the CTAs; a trial drops out at its first non-positive pivot, a
 // trailing sweep is done at its last panel's factorisation, a full sweep
 // after its final phase.  Returns false when a barrier gave up.  The last
 // phase has no barrier when no full sweep runs on (the caller's next fill
 // goes to other matrices or follows a barrier).
-__device__ bool msweep(TrialSet& ts, const CoopArgs& a, Smem& sm)
+__device__ __noinline__ bool msweep(TrialSet& ts, const CoopArgs& a, Smem& sm)
 {
     const int n = a.n;
     const int T = (n + CB - 1) / CB;
-    const bool rec = a.prof && blockIdx.x == 0 && threadIdx.x == 0;
-    for (int t = 0; t < ts.nt; ++t) ts.state[t] = 0;
-    for (int K = 0; K < T; ++K) {
-        const int k0 = K * CB, b = n - k0 < CB ? n - k0 : CB;
-        unsigned long long tp = rec ? global_ns() : 0ull;
-        for (int t = 0; t < ts.nt; ++t)
-            if (ts.state[t] == 0) panel_load(ts.A[t], n, k0, b, sm.pf[t]);
-        __syncthreads();
-        {
-            const int w = threadIdx.x >> 5;
-            if (w < ts.nt && ts.state[w] == 0) panel_chol(sm.pf[w], &sm.pd[w]);
+    unsigned long long* const prof = a.prof;
+    const bool rec = prof && blockIdx.x == 0 && threadIdx.x == 0;
+    const int nt = ts.nt;
+    unsigned run = (1u << nt) - 1u, fullm = 0u, passed = 0u;   // bit t: trial t
+#pragma unroll
+    for (int t = 0; t < NTRIAL; ++t) {
+        if (t >= nt) continue;
+        if (ts.full[t]) fullm |= 1u << t;
+        if (threadIdx.x == 0) sm.A[t] = ts.A[t];
+    }
+    if (threadIdx.x == 0) {
+        sm.Wb = a.Wb;
+        sm.Db = a.Db;
+    }
+    __syncthreads();
+    auto done = [&](bool alive) {
+#pragma unroll
+        for (int t = 0; t < NTRIAL; ++t)
+            if (t < nt) ts.state[t] = (run >> t & 1u) ? 0 : (passed >> t & 1u) ? 1 : -1;
+        return alive;
+    };
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, wt = w & (NTRIAL - 1);   // (a warp's trial)
+    // what a phase loads and works on, set up before the barrier in front of it
+    int total = 0;
+    const double* wpanel = nullptr;
+    TileJob cur;
+    TileAddr addr;
+    int k0 = 0, b = 0;
+    // tiles of a running trial in phase K
+    auto tiles = [&](int K, int t) {
+        const int tt = (run >> t & 1u) ? ((fullm >> t & 1u) ? T : T - K - 1) : 0;
+        return tt * (tt + 1) / 2;
+    };
+    auto job = [&](int K, unsigned started, int q) {
+        TileJob j;
+        int t = 0, r = q;
+#pragma unroll
+        for (int u = 0; u < NTRIAL - 1; ++u) {
+            const int tt = (started >> u & 1u) ? ((fullm >> u & 1u) ? T : T - K - 1) : 0, c = tt * (tt + 1) / 2;
+            if (t == u && r >= c) {
+                r -= c;
+                ++t;
+            }
         }
+        j.trial = t;
+        j.A = sm.A[t];
+        j.full = (fullm >> t & 1u) != 0u;
+        st_decode(r, &j.I, &j.J);
+        if (!j.full) {
+            j.I += K + 1;
+            j.J += K + 1;
+        }
+        return j;
+    };
+    auto wd = [&](int K) { return sm.Wb + (K & 1 ? (unsigned)n * CB : 0u); };
+    auto dd = [&](int K) { return sm.Db + (K & 1 ? CB * CB : 0); };
+    auto setup = [&](int K) {
+        k0 = K * CB;
+        b = n - k0 < CB ? n - k0 : CB;
+        total = 0;
+#pragma unroll
+        for (int t = 0; t < NTRIAL; ++t) total += tiles(K, t);
+        if (run >> wt & 1u)
+            wpanel = sm.A[wt] + ((unsigned)(k0 + (lane >> 2)) * (unsigned)n + (unsigned)(k0 + 2 * (lane & 3)));
+        if ((int)blockIdx.x < total) {
+            cur = job(K, run, blockIdx.x);
+            addr = tile_addr(cur, n, K, k0, b, wd(K + 1), dd(K + 1));
+        }
+    };
+    setup(0);
+    for (int K = 0; K < T; ++K) {
+        unsigned long long tp = rec ? global_ns() : 0ull;
+        const unsigned started = run;
+        const bool wrun = (run >> wt & 1u) != 0u, wfull = (fullm >> wt & 1u) != 0u;
+        // the panel blocks and the CTA's first tile, in one round trip
+        PanelTiles pf;
+        if (wrun && w < NTRIAL) panel_load(wpanel, n, b, pf);
+        TileLoad load;
+        int q = blockIdx.x;
+        if (q < total) tile_load(addr, load);
+        if (wrun && w < NTRIAL) panel_chain(pf, wt, wfull, sm);
+        if (wrun && w >= NTRIAL && wfull) panel_help(wt, sm);
         __syncthreads();
-        bool running = false;
-        int tiles[NTRIAL];
-        int total = 0;
-        for (int t = 0; t < ts.nt; ++t) {
-            tiles[t] = 0;
-            if (ts.state[t] != 0) continue;
+#pragma unroll
+        for (int t = 0; t < NTRIAL; ++t) {
+            if (!(started >> t & 1u)) continue;
             if (!sm.pd[t]) {
-                ts.state[t] = -1;
-            } else if (!ts.full[t] && K == T - 1) {
-                ts.state[t] = 1;
-            } else {
-                running = true;
-                const int tt = ts.full[t] ? T : T - K - 1;
-                tiles[t] = tt * tt;
-                total += tiles[t];
+                run &= ~(1u << t);
+            } else if (!(fullm >> t & 1u) && K == T - 1) {
+                run &= ~(1u << t);
+                passed |= 1u << t;
             }
         }
         if (rec) {
             const unsigned long long tn = global_ns();
-            a.prof[COOP_PROF_FACTOR] += tn - tp;
-            a.prof[COOP_PROF_PHASES] += 1;
+            prof[COOP_PROF_FACTOR] += tn - tp;
+            prof[COOP_PROF_PHASES] += 1;
             tp = tn;
         }
-        if (!running) return true;
-        const double* Wprev = a.Wb + (size_t)((K + 1) & 1) * n * CB;
-        const double* Dprev = a.Db + (size_t)((K + 1) & 1) * CB * CB;
-        double* Wcur = a.Wb + (size_t)(K & 1) * n * CB;
-        double* Dcur = a.Db + (size_t)(K & 1) * CB * CB;
-        for (int q = blockIdx.x; q < total; q += gridDim.x) {
-            int t = 0, r = q;
-            while (r >= tiles[t]) {
-                r -= tiles[t];
-                ++t;
+        if (!run) return done(true);
+        int set = 0;
+        while (q < total) {
+            q += gridDim.x;
+            const TileJob now = cur;
+            TileLoad here = load;
+            if (q < total) {
+                cur = job(K, started, q);
+                tile_load(tile_addr(cur, n, K, k0, b, wd(K + 1), dd(K + 1)), load);
             }
-            if (ts.full[t]) {
-                tile_step<true>(ts.A[t], n, K, k0, b, r % T, r / T, Wprev, Dprev, Wcur, Dcur, sm, sm.pf[t]);
-            } else {
-                const int tt = T - K - 1;
-                tile_step<false>(ts.A[t], n, K, k0, b, K + 1 + r % tt, K + 1 + r / tt, Wprev, Dprev, Wcur, Dcur, sm,
-                                 sm.pf[t]);
-            }
+            if (!(run >> now.trial & 1u)) continue;
+            tile_step(now, n, K, here, wd(K), dd(K), set, sm);
+            if (now.I != K && now.J != K) set ^= 1;   // (a tile with a barrier)
         }
-        if (a.prof) __syncthreads();
-        if (rec) a.prof[COOP_PROF_TILES] += global_ns() - tp;
-        if (!grid_sync(a.bar, sm, a.prof)) return false;
+        if (prof) __syncthreads();
+        if (rec) prof[COOP_PROF_TILES] += global_ns() - tp;
+        if (K + 1 < T) setup(K + 1);
+        if (!grid_sync(sm.bar, sm, prof)) return done(false);
     }
-    for (int t = 0; t < ts.nt; ++t)
-        if (ts.state[t] == 0 && ts.full[t]) {
-            sweep_final(ts.A[t], a, nullptr, nullptr, nullptr, nullptr, 0.0);
-            if (!grid_sync(a.bar, sm, a.prof)) return false;
-            ts.state[t] = 1;
-        }
-    return true;
+    const unsigned fin = run & fullm;   // (at most one)
+    if (fin) {
+        sweep_final(sm.A[__ffs(fin) - 1], a, sm, ts.Xm, ts.Mout, ts.Fout);
+        if (!grid_sync(sm.bar, sm, prof)) return done(false);
+        run &= ~fin;
+        passed |= fin;
+    }
+    return done(true);
+}
+
+// One full sweep: 1 (positive definite), 0 (a non-positive pivot) or -1 (a
+// barrier gave up).
+__device__ int sweep(double* A, const CoopArgs& a, Smem& sm, const double* Xm = nullptr, double* Mout = nullptr,
+                     double* Fout = nullptr)
+{
+    TrialSet ts;
+#pragma unroll
+    for (int t = 0; t < NTRIAL; ++t) {
+        ts.A[t] = A;
+        ts.full[t] = 1;
+    }
+    ts.nt = 1;
+    ts.Xm = Xm;
+    ts.Mout = Mout;
+    ts.Fout = Fout;
+    if (!msweep(ts, a, sm)) return -1;
+    return ts.state[0] == 1 ? 1 : 0;
+}
+
+// The lower tiles of a sweep's matrix: f(i, j) for i, j < n, by the grid in
+// strips of eight rows.
+template <class F>
+__device__ __forceinline__ void lower_fill(int n, F f)
+{
+    const int T = (n + CB - 1) / CB;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int u = blockIdx.x; u < 2 * T * (T + 1); u += gridDim.x) {
+        int I, J;
+        st_decode(u >> 2, &I, &J);
+        const int i = I * CB + CW * (u & 3) + w, j = J * CB + lane;
+        if (i < n && j < n) f(i, j);
+    }
 }
 
 // ---- products ------------------------------------------------------------------
 
+// A thread's four entries of a block: rows warp + 8 j, column lane.
+__device__ __forceinline__ void block_store(Block& m, int j, double v) { m[(threadIdx.x >> 5) + CW * j][threadIdx.x & 31] = v; }
+
 // out = sym(Zi (Diag(-a) X + Diag(-b) Y) + e1 E1 + e2 E2) (b, Y, E2 may be
 // null; the row scales enter negated, -(a_k X_kc) being exactly
-// (-a_k) X_kc): the owner of the tile pair (I, J), (J, I) forms both
-// products and writes the symmetric part.  k in chunks of 32; thread
-// (r, cc) holds P(I0 + r, J0 + c) and P(J0 + c, I0 + r) for c = cc + 8t.
-__device__ void gemm_sym(const double* Zi, const double* av, const double* X, const double* bv, const double* Y,
-                         double e1, const double* E1, double e2, const double* E2, int n, double* out, Smem& sm)
+// (-a_k) X_kc; X, Y, E1, E2 symmetric): the owner of the tile pair (I, J),
+// (J, I) forms both products on the tensor instruction (a warp E tiles of
+// P_IJ and their mirrors of P_JI) and writes the symmetric part.  k in chunks
+// of 32 through two sets of shared-memory operands, the next chunk's loads in
+// flight during a chunk's products.  E = 1: a CTA takes half of a pair's rows
+// of I, for grids of as many CTAs as halves (at n = 343 the 66 pairs would leave
+// half of the chip idle); the sums are the same.
+template <int E>
+__device__ __noinline__ void gemm_sym_e(const double* Zi, const double* av, const double* X, const double* bv,
+                                        const double* Y, double e1, const double* E1, double e2, const double* E2,
+                                        int n, double* out, Smem& sm)
 {
     const int T = (n + CB - 1) / CB;
-    const int tid = threadIdx.x, r = tid % CB, cc = tid / CB;
-    const int npairs = T * (T + 1) / 2;
-    for (int pq = blockIdx.x; pq < npairs; pq += gridDim.x) {
-        int I = 0, rem = pq;
-        while (rem >= T - I) {
-            rem -= T - I;
-            ++I;
-        }
-        const int J = I + rem;
-        const int i0 = I * CB, j0 = J * CB;
-        double acc1[4] = {0.0, 0.0, 0.0, 0.0}, acc2[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int k0 = 0; k0 < n; k0 += CB) {
-            for (int e = tid; e < CB * CB; e += CT) {
-                const int p = e % CB, q = e / CB;
-                const int kk = k0 + q, kb = k0 + p;
-                sm.A1[p][q] = (i0 + p < n && kk < n) ? Zi[(i0 + p) + (size_t)kk * n] : 0.0;
-                sm.A2[p][q] = (j0 + p < n && kk < n) ? Zi[(j0 + p) + (size_t)kk * n] : 0.0;
-                double v1 = 0.0, v2 = 0.0;
-                if (kb < n && j0 + q < n) {
-                    const size_t idx = kb + (size_t)(j0 + q) * n;
-                    v1 = -av[kb] * X[idx];
-                    if (bv) v1 = fma(-bv[kb], Y[idx], v1);
-                }
-                if (kb < n && i0 + q < n) {
-                    const size_t idx = kb + (size_t)(i0 + q) * n;
-                    v2 = -av[kb] * X[idx];
-                    if (bv) v2 = fma(-bv[kb], Y[idx], v2);
-                }
-                sm.V1[p][q] = v1;   // B(k, J0 + q)
-                sm.V2[p][q] = v2;   // B(k, I0 + q)
-            }
-            __syncthreads();
-#pragma unroll 4
-            for (int k = 0; k < CB; ++k) {
-                const double a1 = sm.A1[r][k];
-                const double b2 = sm.V2[k][r];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int r = lane >> 2, c = lane & 3;
+    constexpr int UNITS = E == 2 ? 1 : 2;
+    for (int u = blockIdx.x; u < UNITS * (T * (T + 1) / 2); u += gridDim.x) {
+        int I, J;
+        st_decode(u / UNITS, &I, &J);
+        const int hh = u % UNITS;
+        const int ta = E == 2 ? w >> 1 : 2 * hh + (w >> 2), tb = E == 2 ? 2 * (w & 1) : w & 3;
+        const bool off = I != J;
+        double z[2][4], x[2][4], y[2][4], sa, sb;
+        auto load = [&](int k0) {
+            const int k = k0 + lane;
+            sa = k < n ? -av[k] : 0.0;
+            sb = bv && k < n ? -bv[k] : 0.0;
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const int c = cc + 8 * t;
-                    acc1[t] = fma(a1, sm.V1[k][c], acc1[t]);
-                    acc2[t] = fma(sm.A2[c][k], b2, acc2[t]);
+            for (int side = 0; side < 2; ++side)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int i = (side ? J : I) * CB + w + CW * j;
+                    const bool in = i < n && k < n && (side ? off : !(E == 1 && off && (j >> 1) != hh));
+                    const size_t o = (size_t)i * n + k;
+                    z[side][j] = in ? __ldcg(Zi + o) : 0.0;
+                    x[side][j] = in ? __ldcg(X + o) : 0.0;
+                    y[side][j] = bv && in ? __ldcg(Y + o) : 0.0;
+                }
+        };
+        auto store = [&](int set) {
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                if (side && !off) continue;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    double h = sa * x[side][j];
+                    if (bv) h = fma(sb, y[side][j], h);
+                    block_store(sm.b[4 * set + side], j, z[side][j]);
+                    block_store(sm.b[4 * set + 2 + side], j, h);
                 }
             }
+        };
+        double2 p[E] = {}, pt[E] = {};   // P_IJ (ta, tb + e), P_JI (tb + e, ta)
+        load(0);
+        store(0);
+        __syncthreads();
+        int set = 0;
+        for (int k0 = 0; k0 < n; k0 += CB, set ^= 1) {
+            const bool more = k0 + CB < n;
+            if (more) load(k0 + CB);
+            const Block& zi = sm.b[4 * set];
+            const Block& zj = sm.b[4 * set + (off ? 1 : 0)];
+            const Block& hi = sm.b[4 * set + 2];
+            const Block& hj = sm.b[4 * set + 2 + (off ? 1 : 0)];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const double2 f = frag(zi, ta, q), g = frag(hi, ta, q);
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    mma(p[e], f, frag(hj, tb + e, q));
+                    mma(pt[e], frag(zj, tb + e, q), g);
+                }
+            }
+            if (more) store(set ^ 1);
             __syncthreads();
         }
+        double* scratch = &sm.V(0, 0)[0][0] + 64 * w;
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int i = i0 + r, j = j0 + cc + 8 * t;
-            if (i >= n || j >= n) continue;
-            const size_t ij = i + (size_t)j * n, ji = j + (size_t)i * n;
-            double vij = acc1[t] + e1 * E1[ij];
-            double vji = acc2[t] + e1 * E1[ji];
-            if (E2) {
-                vij += e2 * E2[ij];
-                vji += e2 * E2[ji];
+        for (int e = 0; e < E; ++e) {
+            // P_JI's tile transposed through the warp's scratch
+            scratch[st_elem(2 * c, r)] = pt[e].x;
+            scratch[st_elem(2 * c + 1, r)] = pt[e].y;
+            __syncwarp();
+            const double2 m = st_ld(scratch + st_pair(r, c));
+            __syncwarp();
+            const int i = I * CB + 8 * ta + r;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int j = J * CB + 8 * (tb + e) + 2 * c + k;
+                if (i >= n || j >= n) continue;
+                const size_t ij = (size_t)i * n + j, ji = (size_t)j * n + i;
+                double vij = (k ? p[e].y : p[e].x) + e1 * E1[ij];
+                double vji = (k ? m.y : m.x) + e1 * E1[ij];
+                if (E2) {
+                    vij += e2 * E2[ij];
+                    vji += e2 * E2[ij];
+                }
+                const double v = i == j ? vij : 0.5 * (vij + vji);
+                out[ij] = v;
+                if (off) out[ji] = v;
             }
-            const double v = i == j ? vij : 0.5 * (vij + vji);
-            out[ij] = v;
-            out[ji] = v;
         }
     }
+}
+
+__device__ __forceinline__ void gemm_sym(const double* Zi, const double* av, const double* X, const double* bv,
+                                         const double* Y, double e1, const double* E1, double e2, const double* E2,
+                                         int n, double* out, Smem& sm)
+{
+    const int T = (n + CB - 1) / CB;
+    if (T * (T + 1) <= (int)gridDim.x) gemm_sym_e<1>(Zi, av, X, bv, Y, e1, E1, e2, E2, n, out, sm);
+    else gemm_sym_e<2>(Zi, av, X, bv, Y, e1, E1, e2, E2, n, out, sm);
+}
+
+// sum_c a(c) b(c) over a row, by a warp: the lanes' loads of 12 steps are in
+// flight together (three steps at a time took a round trip to L2 each).
+template <class FA, class FB>
+__device__ __forceinline__ double row_dot(int n, FA fa, FB fb)
+{
+    const int lane = threadIdx.x & 31;
+    double acc = 0.0;
+    for (int c0 = lane; c0 < n; c0 += 32 * 12) {
+        double x[12], y[12];
+#pragma unroll
+        for (int q = 0; q < 12; ++q) {
+            const int c = c0 + 32 * q;
+            x[q] = c < n ? fa(c) : 0.0;
+            y[q] = c < n ? fb(c) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 12; ++q) acc = fma(x[q], y[q], acc);
+    }
+    return warp_sum(acc);
 }
 
 // One warp per row i (the grid's warps in turn): out_i = sum_c F(c, i) v_c
@@ -685,9 +904,7 @@ __device__ void warp_rows_matvec(const double* F, int n, const double* v, double
     const int nw = gridDim.x * CW;
     for (int i = blockIdx.x * CW + (threadIdx.x >> 5); i < n; i += nw) {
         const double* col = F + (size_t)i * n;
-        double acc = 0.0;
-        for (int c = lane; c < n; c += 32) acc = fma(col[c], v ? v[c] : -1.0, acc);
-        acc = warp_sum(acc);
+        const double acc = row_dot(n, [=](int c) { return __ldcg(col + c); }, [=](int c) { return v ? __ldcg(v + c) : -1.0; });
         if (lane == 0) out[i] = acc;
     }
 }
@@ -699,9 +916,7 @@ __device__ void warp_rows_resid(const double* M, int n, const double* b, const d
     const int nw = gridDim.x * CW;
     for (int i = blockIdx.x * CW + (threadIdx.x >> 5); i < n; i += nw) {
         const double* col = M + (size_t)i * n;
-        double acc = 0.0;
-        for (int c = lane; c < n; c += 32) acc = fma(col[c], x[c], acc);
-        acc = warp_sum(acc);
+        const double acc = row_dot(n, [=](int c) { return __ldcg(col + c); }, [=](int c) { return __ldcg(x + c); });
         if (lane == 0) r[i] = (b ? b[i] : -1.0) - acc;
     }
 }
@@ -713,9 +928,7 @@ __device__ void warp_rows_refine(const double* F, int n, const double* r, double
     const int nw = gridDim.x * CW;
     for (int i = blockIdx.x * CW + (threadIdx.x >> 5); i < n; i += nw) {
         const double* col = F + (size_t)i * n;
-        double acc = 0.0;
-        for (int c = lane; c < n; c += 32) acc = fma(col[c], r[c], acc);
-        acc = warp_sum(acc);
+        const double acc = row_dot(n, [=](int c) { return __ldcg(col + c); }, [=](int c) { return __ldcg(r + c); });
         if (lane == 0) {
             t[i] = acc;
             x[i] = x[i] + acc;
@@ -730,9 +943,8 @@ __device__ void warp_rows_rhs(const double* Zi, const double* dX1, const double*
     const int nw = gridDim.x * CW;
     for (int i = blockIdx.x * CW + (threadIdx.x >> 5); i < n; i += nw) {
         const size_t o = (size_t)i * n;
-        double acc = 0.0;
-        for (int c = lane; c < n; c += 32) acc = fma(Zi[o + c] * dX1[o + c], dy1[c], acc);
-        acc = warp_sum(acc);
+        const double acc = row_dot(n, [=](int c) { return __ldcg(Zi + o + c) * __ldcg(dX1 + o + c); },
+                                   [=](int c) { return __ldcg(dy1 + c); });
         if (lane == 0) rhs[i] = mu * Zi[o + i] - acc;
     }
 }
@@ -749,7 +961,7 @@ __device__ bool solve(const CoopArgs& a, const double* F, const double* b, doubl
     return grid_sync(a.bar, sm, a.prof);
 }
 
-__global__ void __launch_bounds__(CT, 1) ipm_coop_kernel(CoopArgs a)
+__global__ void __launch_bounds__(CT, 1) ipm_coop_kernel(const __grid_constant__ CoopArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
@@ -759,30 +971,35 @@ __global__ void __launch_bounds__(CT, 1) ipm_coop_kernel(CoopArgs a)
     const double* __restrict__ L = a.L;
     double* X = a.Xbase + (a.xslot ? (size_t)(*a.xslot) * nn : 0);
     const unsigned long long t_call = a.prof && blockIdx.x == 0 ? global_ns() : 0ull;
+    if (threadIdx.x == 0) {
+        sm.epoch = 0u;
+        sm.bar = a.bar;
+    }
 
     // ---- initial point (src/ipm_mc_pk.c:65-99): y_c = sum_r |L_rc| + 1.1,
     // zd = y - diag(L), X = I; psi = trace(L), mu = sum(zd) / 2n, phi = sum(y)
-    const size_t vstride = (size_t)VCTA * CT;
-    for (int v = blockIdx.x; v < VCTA; v += gridDim.x) {
-        const size_t vt = (size_t)v * CT + threadIdx.x;
+    const int parts = sum_parts(n);
+    const size_t vstride = (size_t)parts * CT;
+    for (int v = blockIdx.x; v < parts; v += gridDim.x) {
         double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-        for (size_t c = vt; c < (size_t)n; c += vstride) {
-            double acc = 0.0;
-            const double* Lc = L + c * n;
-            for (int r = 0; r < n; ++r) acc += fabs(Lc[r]);
-            const double yc = acc + 1.1;
-            const double zc = yc - Lc[c];
-            a.y[c] = yc;
-            a.zd[c] = zc;
-            s0 += Lc[c];
-            s1 += zc;
-            s2 += yc;
+        for (int c = v * CW + (threadIdx.x >> 5); c < n; c += parts * CW) {
+            const double* Lc = L + (size_t)c * n;
+            const double acc = row_dot(n, [=](int q) { return fabs(Lc[q]); }, [](int) { return 1.0; });
+            if ((threadIdx.x & 31) == 0) {
+                const double yc = acc + 1.1;
+                const double zc = yc - Lc[c];
+                a.y[c] = yc;
+                a.zd[c] = zc;
+                s0 += Lc[c];
+                s1 += zc;
+                s2 += yc;
+            }
         }
         block_partials(s0, s1, s2, 0.0, sm, a.part, v);
     }
     for (size_t e = gtid; e < nn; e += gstride) X[e] = (e % n == e / n) ? 1.0 : 0.0;
     bool alive = grid_sync(a.bar, sm, a.prof);
-    grid_totals(a.part, sm);
+    grid_totals(a.part, parts, sm);
     double psi = sm.tot[0];
     double mu = sm.tot[1] / (2.0 * n);
     double phi = sm.tot[2];
@@ -804,13 +1021,12 @@ __global__ void __launch_bounds__(CT, 1) ipm_coop_kernel(CoopArgs a)
         int pd = 1;
         if (!have_zi) {
             // Zi = inv(Z), Z = Diag(zd) - L off the diagonal
-            for (size_t e = gtid; e < nn; e += gstride) {
-                const int i = (int)(e % n), j = (int)(e / n);
-                Zi[e] = i == j ? a.zd[i] : -L[e];
-            }
+            lower_fill(n, [&](int i, int j) {
+                Zi[(size_t)i * n + j] = i == j ? a.zd[i] : -L[i + (size_t)j * n];
+            });
             if (!(alive = grid_sync(a.bar, sm, a.prof))) break;
             // (its last phase also writes M = Zi .* X and F = M)
-            pd = sweep<true>(Zi, a, sm, X, a.M, F);
+            pd = sweep(Zi, a, sm, X, a.M, F);
             if (pd < 0) {
                 alive = false;
                 break;
@@ -829,7 +1045,7 @@ __global__ void __launch_bounds__(CT, 1) ipm_coop_kernel(CoopArgs a)
         }
         have_zi = false;
         // F = inv(M); dy1 = F (-e)
-        pd = sweep<true>(F, a, sm);
+        pd = sweep(F, a, sm);
         if (pd < 0) {
             alive = false;
             break;
@@ -895,12 +1111,12 @@ __global__ void __launch_bounds__(CT, 1) ipm_coop_kernel(CoopArgs a)
                 if (di + 1 < IPM_MAX_TRIALS) add(F, ad * 0.8, true, false);
             }
             // (dy_i = dy1_i + dy2_i)
-            for (size_t e = gtid; e < nn; e += gstride) {
-                const int i = (int)(e % n), j = (int)(e / n);
+            lower_fill(n, [&](int i, int j) {
+                const size_t e = (size_t)i * n + j;
                 for (int t = 0; t < ts.nt; ++t)
-                    ts.A[t][e] = dual[t] ? (i == j ? fma(alpha[t], a.dy1[i] + a.dy2[i], a.zd[i]) : -L[e])
+                    ts.A[t][e] = dual[t] ? (i == j ? fma(alpha[t], a.dy1[i] + a.dy2[i], a.zd[i]) : -L[i + (size_t)j * n])
                                          : fma(alpha[t], a.dX[e], X[e]);
-            }
+            });
             if (!(alive = grid_sync(a.bar, sm, a.prof))) break;
             if (!(alive = msweep(ts, a, sm))) break;
             // each search: the first of its trials that passed, in order
@@ -939,11 +1155,16 @@ __global__ void __launch_bounds__(CT, 1) ipm_coop_kernel(CoopArgs a)
         // zd += ad dy (dy = dy1 + dy2), and the sums zx = <Z, X>, lx = <L, X>,
         // sum(y) of the new point.  The diagonal of X goes with the vectors
         // (the thread that moves zd_i also moves X_ii).
-        for (int v = blockIdx.x; v < VCTA; v += gridDim.x) {
+        for (int v = blockIdx.x; v < parts; v += gridDim.x) {
             const size_t vt = (size_t)v * CT + threadIdx.x;
             double zx = 0.0, lx = 0.0, ys = 0.0;
-            for (size_t e = vt; e < nn; e += vstride) {
-                const int i = (int)(e % n), j = (int)(e / n);
+            int i = (int)(vt % n), j = (int)(vt / n);
+            const int di = (int)(vstride % n), dj = (int)(vstride / n);
+            for (size_t e = vt; e < nn; e += vstride, i += di, j += dj) {
+                if (i >= n) {
+                    i -= n;
+                    ++j;
+                }
                 if (i == j) continue;
                 const double xv = fma(ap, a.dX[e], X[e]);
                 X[e] = xv;
@@ -967,7 +1188,7 @@ __global__ void __launch_bounds__(CT, 1) ipm_coop_kernel(CoopArgs a)
             block_partials(zx, lx, ys, 0.0, sm, a.part, v);
         }
         if (!(alive = grid_sync(a.bar, sm, a.prof))) break;
-        grid_totals(a.part, sm);
+        grid_totals(a.part, parts, sm);
         mu = sm.tot[0] / (2.0 * n);
         if (ap + ad > 1.6) mu *= 0.5;
         if (ap + ad > 1.9) mu *= 0.2;
@@ -1020,7 +1241,7 @@ unsigned long long* coop_prof_device()
 
 // The per-size schedule: the grid (CTAs) to use for T = ceil(n / 32) tiles
 // per dimension, filled by the autotuner (bqb_ipm_autotune) or set by hand
-// (bqb_ipm_schedule_set); sizes without an entry use one CTA per tile.
+// (bqb_ipm_schedule_set); sizes without an entry use coop_config's rule.
 std::mutex g_sched_mu;
 std::map<int, int> g_sched;
 
@@ -1034,8 +1255,8 @@ std::atomic<int> g_large_share{0};
 
 namespace {
 
-// Grid size for n: the schedule's entry for its tile count, else one CTA
-// per 32 x 32 tile of the sweep; at most as many as can be co-resident (one
+// Grid size for n: the schedule's entry for its tile count, else one CTA for
+// half a pair of 32 x 32 tiles (and the whole chip from 7/8 of it on); at most as many as can be co-resident (one
 // per SM at this register count), divided by the number of engines bounding
 // large nodes at the time.
 CoopConfig coop_config(int n)
@@ -1052,7 +1273,7 @@ CoopConfig coop_config(int n)
         ready.store(1);
     }
     const int T = (n + CB - 1) / CB;
-    int g = T * T;
+    int g = 8 * T * (T + 1) >= 7 * max_blocks ? max_blocks : T * (T + 1);
     {
         std::lock_guard<std::mutex> lock(g_sched_mu);
         auto it = g_sched.find(T);
