@@ -36,7 +36,11 @@ kgon_sa_kernel(const double* __restrict__ X, int n, int K, int types, int chains
     __syncthreads();
     const int c = blockIdx.x * SA_WARPS + w;
     if (c >= chains) return;
-    kgon_chain_warp(Xs, n, K, types, c, seed, sT[0], P, cost_out, perm_out, status);
+    if (x_in_smem)
+        kgon_chain_warp([=](unsigned i) { return sa_smem[i]; }, n, K, types, c, seed, sT[0], P, cost_out, perm_out,
+                        status);
+    else
+        kgon_chain_warp([=](unsigned i) { return X[i]; }, n, K, types, c, seed, sT[0], P, cost_out, perm_out, status);
 }
 
 }  // namespace
