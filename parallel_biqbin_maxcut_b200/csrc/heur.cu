@@ -20,6 +20,7 @@
 
 #include "cta_linalg.cuh"
 #include "heur.cuh"
+#include "sym_tiles.cuh"
 
 namespace bqb {
 
@@ -42,6 +43,12 @@ __global__ void __launch_bounds__(POTRF_THREADS) potrf_kernel(double* Z, int n, 
     if (in_smem && ok) {
         for (size_t e = threadIdx.x; e < nn; e += blockDim.x) Z[e] = A[e];
     }
+    if (threadIdx.x == 0) *status = ok ? 0 : 1;
+}
+
+__global__ void __launch_bounds__(ST_THREADS) potrf_tiles_kernel(double* Z, int n, int* status)
+{
+    const bool ok = st_potrf(Z, n, st_smem);
     if (threadIdx.x == 0) *status = ok ? 0 : 1;
 }
 
@@ -188,6 +195,14 @@ __global__ void select_kernel(const double* __restrict__ vals, int count, const 
 
 void potrf_device(double* dZ, int n, int* dstatus, cudaStream_t s)
 {
+    if (n <= ST_NMAX) {   // (what both take is at st_potrf)
+        const size_t bytes = (st_buffers(st_tiles(n)) + 1) * sizeof(double);
+        BQB_SMEM_LIMIT(potrf_tiles_kernel, bytes);
+        potrf_tiles_kernel<<<1, ST_THREADS, bytes, s>>>(dZ, n, dstatus);
+        BQB_COUNT_LAUNCH();
+        check_launch("potrf_tiles_kernel");
+        return;
+    }
     const size_t need = ((size_t)((n + 1) & ~1) + (size_t)n * n) * sizeof(double);
     const int in_smem = need <= rt().smem_optin ? 1 : 0;
     const size_t bytes = in_smem ? need : (size_t)((n + 1) & ~1) * sizeof(double);

@@ -34,7 +34,6 @@
 #include <math.h>
 
 #include "bundle_body.cuh"
-#include "cta_linalg.cuh"
 #include "cuts.cuh"
 #include "ipm_reg_body.cuh"
 #include "kgon_sa.cuh"
@@ -478,8 +477,7 @@ __device__ __noinline__ double nk_heuristic(const FusedCfg& c, Nk& k)
     const size_t nn = (size_t)n * n;
     const int nv = (n + 1) & ~1;
     double* Zs = smem;
-    double* colb = Zs + nn;
-    double* dg = colb + nv;
+    double* dg = Zs + ((nn + 1) & ~(size_t)1);
     double* wbuf = dg + nv;   // per warp: Lx[nv], x[nv] (as int)
     if (tid == 0) nk_si[5] = 0;
 
@@ -505,7 +503,7 @@ __device__ __noinline__ double nk_heuristic(const FusedCfg& c, Nk& k)
     while (done < 2 && rounds < NK_MAX_GW_ROUNDS) {
         ++done;
         ++rounds;
-        if (!cta_potrf_lower(Zs, n, n, colb)) {
+        if (!st_potrf(Zs, n, wbuf)) {   // (1-opt's buffers are free)
             k.status |= NKS_HEUR;
             __syncthreads();
             return heur_val;
@@ -1530,8 +1528,9 @@ size_t nk_smem_bytes(int N0, int T, int bcap, size_t smem_optin)
     up(ipm_st_smem_doubles_upto(N0, (smem_optin - NK_STATIC_SMEM) / sizeof(double)) * sizeof(double));
     // lambda_eta
     up(le_smem_bytes(bcap < QP_SMEM_K ? bcap : QP_SMEM_K) + 3 * (size_t)bcap * sizeof(double));
-    // heuristic: Z, column buffer, d, 16 warps x (Lx, x)
-    up((nn + 2 * nv + (size_t)(NKT / 32) * 2 * nv) * sizeof(double));
+    // heuristic: Z, d, then the factorisation's buffers or 16 warps x (Lx, x)
+    const size_t fac = st_buffers(st_tiles(N0)) + 1, opt = (size_t)(NKT / 32) * 2 * nv;
+    up((nn + 1 + nv + (fac > opt ? fac : opt)) * sizeof(double));
     // triangle separation: X^T, then the heap
     up(nn * sizeof(double));
     const size_t Tr = T > 0 ? T : 1;

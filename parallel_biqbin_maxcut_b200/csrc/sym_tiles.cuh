@@ -355,8 +355,10 @@ __device__ __forceinline__ bool st_inverse(int T, double* buf, int* flag, Fill f
 // Step j: column j of D and row j of Y go to the lanes by shuffles while the
 // pivot's reciprocal square root is computed, and every lane computes the next
 // pivot for itself, so the chain is eight times a reciprocal square root, a
-// product and an FMA (69 + 8 + 8 cycles) and no shuffle is in it.
-__device__ __forceinline__ bool st_chol_inv(double2 d, double2& y)
+// product and an FMA (69 + 8 + 8 cycles) and no shuffle is in it.  WITH_L: L
+// itself, too.
+template <bool WITH_L = false>
+__device__ __forceinline__ bool st_chol_inv(double2 d, double2& y, double2* l = nullptr)
 {
     const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
     const int row0 = lane & ~3;
@@ -383,6 +385,11 @@ __device__ __forceinline__ bool st_chol_inv(double2 d, double2& y)
         const double le = e * rs;
         p = fma(-le, le, pn);
         const double lr = r > j ? dr * rs : 0.0;
+        if (WITH_L) {
+            const double lj = r >= j ? dr * rs : 0.0;
+            l->x = 2 * c == j ? lj : l->x;
+            l->y = 2 * c + 1 == j ? lj : l->y;
+        }
         d.x = fma(-lr, d0 * rs, d.x);
         d.y = fma(-lr, d1 * rs, d.y);
         const double w0 = y0 * rs, w1 = y1 * rs;
@@ -401,9 +408,14 @@ __device__ __forceinline__ bool st_chol_inv(double2 d, double2& y)
 // same operand twice), the long ones first.
 //
 // `fill(I, J, r, c)` gives -A's pair (row r, columns 2c and 2c + 1 of tile
-// (I, J)), I >= J.  buf, flag, result as for st_inverse.
-template <class Fill>
-__device__ __forceinline__ bool st_posdef(int T, double* buf, int* flag, Fill fill)
+// (I, J)), I >= J.  buf, flag, result as for st_inverse.  FACTOR: `store(I, J,
+// v)` takes the factor's pairs (tiles I >= J) as they come, also in front of a
+// non-positive pivot; without it nothing is stored.
+struct StNoStore {
+    __device__ void operator()(int, int, const double2&) const {}
+};
+template <bool FACTOR = false, class Fill, class Store = StNoStore>
+__device__ __forceinline__ bool st_posdef(int T, double* buf, int* flag, Fill fill, Store store = {})
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = lane >> 2, c = lane & 3;
@@ -420,8 +432,9 @@ __device__ __forceinline__ bool st_posdef(int T, double* buf, int* flag, Fill fi
         st_bar_sync(ST_BAR_P + 1, NC);
         double2 d = st_ld(Pb + 128 + 64 + pr);
         for (int K = 0; K < T; ++K) {
-            double2 y;
-            const bool pd = st_chol_inv(d, y);
+            double2 y, l = make_double2(0.0, 0.0);
+            const bool pd = st_chol_inv<FACTOR>(d, y, &l);
+            if (FACTOR) store(K, K, l);
             failed = pd ? 0 : 1;
             if (lane == 0 && !pd) *flag = K + 1;   // (the panel: an update warp may be one behind)
             st_st(Lb + 64 * (K & 1) + pr, y.x, y.y);
@@ -470,6 +483,7 @@ __device__ __forceinline__ bool st_posdef(int T, double* buf, int* flag, Fill fi
             if (I > K) {
                 st_mma_split(v, nx, st_ld(Lb + 64 * (K & 1) + pr));
                 st_st(V + 64 * I + pr, v.x, v.y);
+                if (FACTOR) store(I, K, v);
             }
             st_bar_sync(ST_BAR_U, NU);
             // the update, four tiles at a time: their operands, their first
@@ -506,6 +520,31 @@ __device__ __forceinline__ bool st_posdef(int T, double* buf, int* flag, Fill fi
         if (!stopped) st_bar_sync(ST_BAR_L + ((T - 1) & 1), NC);
     }
     return __syncthreads_or(failed) == 0;
+}
+
+// The Cholesky factor of the n x n matrix A (column-major, n <= 128, lower
+// triangle read and written; the upper one is left alone) by the CTA; false, in
+// all threads, on a non-positive pivot (then the lower triangle is partly
+// written).  buf: st_buffers(ceil(n / 8)) + 1 doubles of shared memory, 16-byte
+// aligned.  n = 100: 22 us; a column, a barrier and a rank-1 update at a time
+// (cta_potrf_lower) 98.
+static __device__ __noinline__ bool st_potrf(double* A, int n, double* buf)
+{
+    const int T = st_tiles(n), lane = threadIdx.x & 31;
+    return st_posdef<true>(
+        T, buf, reinterpret_cast<int*>(buf + st_buffers(T)),
+        [=](int I, int J, int r, int c) {
+            const int i = 8 * I + r, j = 8 * J + 2 * c;
+            double2 v = make_double2(i == j ? 1.0 : 0.0, i == j + 1 ? 1.0 : 0.0);
+            if (i < n && j < n) v.x = A[i >= j ? i + j * n : j + i * n];
+            if (i < n && j + 1 < n) v.y = A[i >= j + 1 ? i + (j + 1) * n : j + 1 + i * n];
+            return make_double2(-v.x, -v.y);
+        },
+        [=](int I, int J, const double2& v) {
+            const int i = 8 * I + (lane >> 2), j = 8 * J + 2 * (lane & 3);
+            if (i < n && j <= i) A[i + j * n] = v.x;
+            if (i < n && j + 1 <= i) A[i + (j + 1) * n] = v.y;
+        });
 }
 
 }  // namespace bqb
