@@ -52,26 +52,26 @@ void ensure_round_buffers(HeurState& st, int n, int N0, int num)
     st.hstat.ensure(2);
 }
 
-// Hyperplanes v_i = rand()/RAND_MAX - 0.5, count-major (src/heuristic.c:142-143).
-void draw_hyperplanes(HeurState& st, Rng& rng, int n, int num, cudaStream_t s)
-{
-    double* hv = st.hV.ensure((size_t)num * n);
-    for (int c = 0; c < num; ++c)
-        for (int i = 0; i < n; ++i) hv[(size_t)c * n + i] = ((double)rng.next() / (double)(RAND_MAX)) - 0.5;
-    BQB_CUDA(cudaMemcpyAsync(st.V.p, hv, (size_t)num * n * sizeof(double), cudaMemcpyHostToDevice, s));
-}
-
-// Run one GW round on the factor already in st.Z; copy the best cut to x.
+// Run one GW round on the factor in st.Z; copy the best cut to x.  Hyperplanes
+// v_i = rand()/RAND_MAX - 0.5, count-major (src/heuristic.c:142-143).  factored:
+// the factorisation may still run (the host draws meanwhile) and its status is
+// in st.status; it is read with the round's results, and *ok = false when it
+// failed.
 double gw_round_host(HeurState& st, Rng& rng, const double* dPL, int n, const double* dP0L, int N0, int num,
-                     int* x, cudaStream_t s)
+                     int* x, cudaStream_t s, bool factored = false, bool* ok = nullptr)
 {
-    draw_hyperplanes(st, rng, n, num, s);
-    BQB_CUDA(cudaMemsetAsync(st.status.p, 0, 2 * sizeof(int), s));
-    gw_round_device(st, dPL, n, dP0L, N0, num, s);
+    if (!factored) BQB_CUDA(cudaMemsetAsync(st.status.p, 0, 2 * sizeof(int), s));
+    double* hv = st.hV.ensure((size_t)num * n);
+    for (size_t q = 0; q < (size_t)num * n; ++q) hv[q] = ((double)rng.next() / (double)(RAND_MAX)) - 0.5;
+    BQB_CUDA(cudaMemcpyAsync(st.V.p, hv, (size_t)num * n * sizeof(double), cudaMemcpyHostToDevice, s));
+    gw_cuts_device(st, dPL, n, num, s);
+    gw_best_device(st, n, dP0L, N0, num, s);
     BQB_CUDA(cudaMemcpyAsync(st.hbest.p, st.best.p, (size_t)N0 * sizeof(int), cudaMemcpyDeviceToHost, s));
     BQB_CUDA(cudaMemcpyAsync(st.hval.p, st.bestval.p, sizeof(double), cudaMemcpyDeviceToHost, s));
     BQB_CUDA(cudaMemcpyAsync(st.hstat.p, st.status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     BQB_CUDA(cudaStreamSynchronize(s));
+    if (ok) *ok = st.hstat.p[0] == 0;
+    if (ok && !*ok) return -BIG_NUMBER;
     if (st.hstat.p[1]) fatal("GW_heuristic", "1-opt did not terminate");
     if (num > 0) memcpy(x, st.hbest.p + 1, (size_t)(N0 - 1) * sizeof(int));
     return num > 0 ? st.hval.p[0] : -BIG_NUMBER;
@@ -89,7 +89,8 @@ double gw_round_batched(HeurState& st, Rng& rng, const double* dPL, int n, const
     BQB_CUDA(cudaMemsetAsync(st.status.p, 0, 2 * sizeof(int), s));
     const cudaError_t e = gw_project_tf32(st.Z.p, n, H, seed, st.x.p, st.Vf, st.tcerr, s);
     if (e != cudaSuccess) fatal("GW_heuristic (batched projection)", cudaGetErrorString(e));
-    gw_round_finish(st, dPL, n, dP0L, N0, H, s);
+    one_opt_device(st, dPL, n, H, s);
+    gw_best_device(st, n, dP0L, N0, H, s);
     int terr = 0;
     BQB_CUDA(cudaMemcpyAsync(st.hbest.p, st.best.p, (size_t)N0 * sizeof(int), cudaMemcpyDeviceToHost, s));
     BQB_CUDA(cudaMemcpyAsync(st.hval.p, st.bestval.p, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -147,15 +148,23 @@ double heuristic_device(HeurState& st, Rng& rng, const double* dX, const double*
     double heur_val = -BIG_NUMBER;
     while (done < 2) {
         ++done;
+        BQB_CUDA(cudaMemsetAsync(st.status.p, 0, 2 * sizeof(int), s));
         potrf_device(st.Z.p, n, st.status.p, s);
-        BQB_CUDA(cudaMemcpyAsync(st.hstat.p, st.status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-        BQB_CUDA(cudaStreamSynchronize(s));
-        if (st.hstat.p[0]) {
+        bool ok = true;
+        double v = heur_val;
+        if (hyperplanes > 0) {
+            BQB_CUDA(cudaMemcpyAsync(st.hstat.p, st.status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+            BQB_CUDA(cudaStreamSynchronize(s));
+            ok = st.hstat.p[0] == 0;
+            if (ok) v = gw_round_batched(st, rng, dPL, n, dP0L, N0, num, x, s);
+        } else {
+            v = gw_round_host(st, rng, dPL, n, dP0L, N0, num, x, s, true, &ok);
+        }
+        if (!ok) {
             fatal("runHeuristic_unpacked", "Problem with Cholesky factorization");
             return heur_val;
         }
-        heur_val = hyperplanes > 0 ? gw_round_batched(st, rng, dPL, n, dP0L, N0, num, x, s)
-                                   : gw_round_host(st, rng, dPL, n, dP0L, N0, num, x, s);
+        heur_val = v;
         if (heur_val > fh) {
             done = 0;
             fh = heur_val;
@@ -165,9 +174,9 @@ double heuristic_device(HeurState& st, Rng& rng, const double* dX, const double*
             xh[n - 1] = -1.0;
         }
         const double c = 0.3 + 0.6 * ((double)rng.next() / (double)(RAND_MAX));
+        // (xh is written again only after the next round's synchronisation)
         BQB_CUDA(cudaMemcpyAsync(dxh.p, xh.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice, s));
         remix_device(st.Z.p, dX, dxh.p, c, n, s);
-        BQB_CUDA(cudaStreamSynchronize(s));   // xh is reused on the host
     }
     return heur_val;
 }

@@ -30,16 +30,13 @@ void potrf_device(double* dZ, int n, int* dstatus, cudaStream_t s);
 // Z = (1 - c) X + c xh xh^T on the lower triangle (src/heuristic.c:105-110).
 void remix_device(double* dZ, const double* dX, const double* dxh, double c, int n, cudaStream_t s);
 
-// One GW round (src/heuristic.c:119-186) with the factor already in st.Z and
-// the hyperplanes in st.V:  sign(L v) per hyperplane, 1-opt on P_L, lift with
-// the node's fixed variables, evaluate on P0_L, keep the first best.
-// Results: st.best (device), st.bestval (device).
-void gw_round_device(HeurState& st, const double* dPL, int n, const double* dP0L, int N0, int num,
-                     cudaStream_t s);
+// A GW round (src/heuristic.c:119-186) with the factor already in st.Z.  The cuts
+// of the num hyperplanes in st.V: sign(L v), then 1-opt on P_L.
+void gw_cuts_device(HeurState& st, const double* dPL, int n, int num, cudaStream_t s);
 
-// The steps of a GW round after the projection (cuts already in st.x):
-// 1-opt, lift, evaluate, keep the first best.
-void gw_round_finish(HeurState& st, const double* dPL, int n, const double* dP0L, int N0, int num, cudaStream_t s);
+// The round's end, with num cuts in st.x: lift with the node's fixed variables,
+// evaluate on P0_L, keep the first best.  Results: st.best, st.bestval (device).
+void gw_best_device(HeurState& st, int n, const double* dP0L, int N0, int num, cudaStream_t s);
 
 // Batched rounding on the tensor cores (csrc/gw_tc.cu): x[h * n + i] =
 // sign((Lf v_h)_i) for H hyperplanes drawn on the device from `seed`, Lf the
