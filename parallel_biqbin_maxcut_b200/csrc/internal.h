@@ -19,7 +19,7 @@ namespace bqb {
 void ipm_device(DevBuf<double>& ws, const double* dL, double* dX, int n, double* dout, cudaStream_t s,
                 const int* xslot = nullptr, double* yout = nullptr);
 
-// Largest n of the register-resident IPM body (RM_NMAX in reg_linalg.cuh);
+// Largest n of the one-CTA IPM body (ST_NMAX in sym_tiles.cuh);
 // ipm_device hands larger problems to ipm_large.
 constexpr int IPM_REG_NMAX = 128;
 

@@ -1,5 +1,5 @@
 // The basic SDP interior-point method (src/ipm_mc_pk.c:28-359) for n above
-// the register-resident limit (IPM_REG_NMAX = 128): ONE cooperative launch
+// the one-CTA limit (IPM_REG_NMAX = 128): ONE cooperative launch
 // per call.  Every CTA (one per SM at most) runs the whole predictor-
 // corrector loop; the phases of an iteration (the inverses, the solves, the
 // two products, the line searches' positive-definiteness tests, the step)
@@ -36,19 +36,19 @@
 // round trip to L2 1600 (the panel block, and the CTA's first tile and its panel
 // columns, are loaded together, from addresses worked out before the barrier),
 // the panel block's chain of 32 pivots on one warp 6000, a tile 4000.  A call at
-// n = 343 takes 3.8 ms, at n = 150 1.7 ms (with rank-1 panel factors by rows,
-// tiles on the vector pipe and every tile of both triangles 10.2 and 4.1).  All
-// products go through the FP64 tensor instruction as X Y^T of 8 x 8 tiles in
-// its accumulators' layout (a lane's pair of columns is also its operand of
-// the two k = 4 steps); V comes from L by tile columns, each solve with a
-// diagonal tile's inverse and one correction.
+// n = 343 takes 3.8 ms, at n = 150 1.7 (with rank-1 panel factors by rows, scalar
+// tiles and all tiles of both triangles 10.2 and 4.1).  All products go through
+// the FP64 tensor instruction as X Y^T of 8 x 8 tiles in its accumulators' layout
+// (a lane's pair of columns is also its operand of the two k = 4 steps); V comes
+// from L by tile columns, each solve with a diagonal tile's inverse.
 //
 // Each solve with M is the product with F = inv(M) followed by one step of
 // iterative refinement with M = Zi .* X (x <- x + F (b - M x)).
 //
-// The grid barrier is a growing counter in global memory; every wait is bounded (2 s), after which the barrier sets an error word,
-// no CTA waits any more, every loop ends, and the call reports status
-// IPM_SYNC (a fatal error on the host).
+// The grid barrier is a growing counter in global memory; every wait is
+// bounded (2 s), after which the barrier sets an error word, no CTA waits any
+// more, every loop ends, and the call reports status IPM_SYNC (a fatal error on
+// the host).
 #include <math.h>
 
 #include <map>

@@ -14,7 +14,7 @@
 // the batch is done.
 //
 // The phases run the same device code as the engine path where that code
-// is a CTA body: the register-resident IPM (ipm_reg_body.cuh), lambda_eta
+// is a CTA body: the tile IPM (ipm_reg_body.cuh), lambda_eta
 // and the bundle step (bundle_body.cuh), the cut operators (cuts.cuh) and
 // the annealing chains (kgon_sa.cuh), with the same thread count, so the
 // arithmetic is the same.  Triangle separation restates trisep.cu's passes

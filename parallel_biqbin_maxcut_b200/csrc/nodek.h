@@ -108,7 +108,7 @@ struct FusedCfg {
     size_t off[NK_COUNT];
 };
 
-// Largest N0 the fused kernel handles (register-resident IPM).
+// Largest N0 the fused kernel handles (one-CTA IPM).
 constexpr int NK_NMAX = 128;
 
 // Shared-memory bytes the fused kernel needs for problems up to N0 with
