@@ -70,7 +70,8 @@ double gw_round_host(HeurState& st, Rng& rng, const double* dPL, int n, const do
     BQB_CUDA(cudaMemcpyAsync(st.hval.p, st.bestval.p, sizeof(double), cudaMemcpyDeviceToHost, s));
     BQB_CUDA(cudaMemcpyAsync(st.hstat.p, st.status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     BQB_CUDA(cudaStreamSynchronize(s));
-    if (ok) *ok = st.hstat.p[0] == 0;
+    // (1: the factorisation failed; 2: a 1-opt stopped at its flip limit, whose cut counts like any other)
+    if (ok) *ok = (st.hstat.p[0] & 1) == 0;
     if (ok && !*ok) return -BIG_NUMBER;
     if (st.hstat.p[1]) fatal("GW_heuristic", "1-opt did not terminate");
     if (num > 0) memcpy(x, st.hbest.p + 1, (size_t)(N0 - 1) * sizeof(int));
