@@ -17,6 +17,7 @@ namespace bqb {
 // ---------------------------------------------------------------------------
 void fatal(const char* where, const char* msg);
 void set_error(const char* where, const char* msg);
+bool abort_returns();   // a hook is set, so fatal() comes back
 
 #define BQB_CUDA(call)                                                        \
     do {                                                                      \

@@ -153,11 +153,15 @@ double heuristic_device(HeurState& st, Rng& rng, const double* dX, const double*
         potrf_device(st.Z.p, n, st.status.p, s);
         bool ok = true;
         double v = heur_val;
-        if (hyperplanes > 0) {
+        if (hyperplanes > 0 || abort_returns()) {
+            // Draws cannot be taken back: a caller that lives on after a failed
+            // factorisation finds rand() where it stood before this round.
             BQB_CUDA(cudaMemcpyAsync(st.hstat.p, st.status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
             BQB_CUDA(cudaStreamSynchronize(s));
             ok = st.hstat.p[0] == 0;
-            if (ok) v = gw_round_batched(st, rng, dPL, n, dP0L, N0, num, x, s);
+            if (ok)
+                v = hyperplanes > 0 ? gw_round_batched(st, rng, dPL, n, dP0L, N0, num, x, s)
+                                    : gw_round_host(st, rng, dPL, n, dP0L, N0, num, x, s);
         } else {
             v = gw_round_host(st, rng, dPL, n, dP0L, N0, num, x, s, true, &ok);
         }

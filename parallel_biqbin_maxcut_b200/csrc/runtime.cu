@@ -56,6 +56,8 @@ void set_error(const char* where, const char* msg)
 
 thread_local bool t_pool_worker = false;
 
+bool abort_returns() { return g_abort_hook != nullptr; }
+
 void fatal(const char* where, const char* msg)
 {
     set_error(where, msg);
