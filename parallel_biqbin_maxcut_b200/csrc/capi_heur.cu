@@ -179,7 +179,8 @@ double heuristic_device(HeurState& st, Rng& rng, const double* dX, const double*
             xh[n - 1] = -1.0;
         }
         const double c = 0.3 + 0.6 * ((double)rng.next() / (double)(RAND_MAX));
-        // (xh is written again only after the next round's synchronisation)
+        if (done == 2) break;   // (no round follows; the draw of c belongs to the stream)
+        // (xh is written or freed only after the next round's synchronisation)
         BQB_CUDA(cudaMemcpyAsync(dxh.p, xh.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice, s));
         remix_device(st.Z.p, dX, dxh.p, c, n, s);
     }

@@ -1,7 +1,8 @@
 """What a caller of the rounding sees besides its cut: a local search that stops
 at its flip limit (an asymmetric P_L makes two vertices flip for ever; the
-rounding then goes on with the cuts it has), and the rand() state after a failed
-factorisation (src/heuristic.c:38-39, 68-74: only the random cut was drawn)."""
+rounding then goes on with the cuts it has), the rand() state after a failed
+factorisation (src/heuristic.c:38-39, 68-74: only the random cut was drawn), and
+the work left on the device at the return (none)."""
 import ctypes as C
 import os
 import subprocess
@@ -76,3 +77,18 @@ def test_failed_factorisation_leaves_the_random_numbers(lib, lib_globals, hook):
     for _ in range(n):   # the random cut
         libc.rand()
     assert after == libc.rand()
+
+
+@pytest.mark.gpu
+def test_nothing_is_launched_after_the_last_round(lib, lib_globals):
+    SPL, L = _problem(40)
+    n = L.shape[0]
+    lib_globals["X"][: n * n] = _lib.colmajor(O.ipm_mc_pk(L).X)
+    libc.srand(7)
+    before = lib.bqb_kernel_launches()
+    v, x = _round(lib, SPL, L)
+    launches = lib.bqb_kernel_launches() - before
+    # the random cut's value; a round: factor, project, 1-opt, evaluate, select;
+    # a re-mix of Z between two rounds
+    assert launches % 6 == 0 and launches >= 12
+    assert v == O.evaluateSolution(SPL, x)
