@@ -721,8 +721,8 @@ __device__ __noinline__ double nk_trisep(const FusedCfg& c, Nk& k, const double*
         if (tid == 0) nk_si[6] = T > 0 ? (int)V : 0;
     } else {
         if (tid == 0) nk_si[6] = T;
-        if (!(tr_smem_bytes(T) <= c.smem_bytes && tr_replay_cta(k.tscand, V, T, k.tslist, smem)) && warp == 0)
-            tr_replay_warp(k.tscand, V, T, k.tslist, smem);
+        if (tr_smem_bytes(T) <= c.smem_bytes) tr_replay_cta(k.tscand, V, T, k.tslist, smem);
+        else if (warp == 0) tr_replay_warp(k.tscand, V, T, k.tslist, smem);
     }
     __syncthreads();
     *size = nk_si[6];

@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(TR_THREADS) tri_replay_kernel(const TriCand* _
         return;
     }
     if (threadIdx.x == 0) *out_size = T;
-    if (whole && tr_replay_cta(cand, V, T, list, hsm)) return;
-    if (threadIdx.x < 32) tr_replay_warp(cand, V, T, list, hsm);
+    if (whole) tr_replay_cta(cand, V, T, list, hsm);
+    else if (threadIdx.x < 32) tr_replay_warp(cand, V, T, list, hsm);
 }
 
 }  // namespace
@@ -222,7 +222,9 @@ double trisep_device(TriSepState& st, const double* dX, int n, int tri_ineq, dou
     tri_scan_kernel<true><<<blocks, 256, 0, s>>>(dX, XT, n, P, violated, cnt, cand, misc);
     BQB_COUNT_LAUNCH();
     // the CTA-wide replay where its two lists fit in shared memory (T up to
-    // 6300 on a B200; at T = 5000, n = 343 1.6 ms against 46)
+    // 6296 on a B200; at T = 5000, n = 343 1.6 ms against 46, and 6 to 16 against
+    // 86 to 98 for a random X of multiples of 1/8 to 1/65536, where most values
+    // equal others)
     const int Tr = tri_ineq > 0 ? tri_ineq : 1;
     const int whole = tr_smem_bytes(Tr) <= rt().smem_optin ? 1 : 0;
     const size_t bytes = whole ? tr_smem_bytes(Tr) : (size_t)Tr * (sizeof(double) + sizeof(int));

@@ -17,11 +17,14 @@
 //    smallest of L and the chunk's taken candidates together.
 // So a chunk is a merge sort of its candidates (which counts the earlier larger
 // ones on the way), a merge with the sorted list, and pointer jumping along
-// "took the slot of" within the chunk.  Equal values among the removed ones
-// would make the second fact ambiguous (the lowest slot goes first): then the
-// caller replays everything one cut at a time.  A whole separation at n = 343,
-// T = 5000 takes 1.6 ms instead of 46; what bounds the replay is the chunk's
-// chain of CTA barriers and the read of the candidates by one SM.
+// "took the slot of" within the chunk.  Equal values leave in the order of their
+// slots, and all of them are in the list before the first one leaves (a cut
+// equal to the minimum is not taken): the list is kept in the order of (value,
+// slot), and where a taken candidate equals another value of the union the slots
+// are found run by run in ascending order instead, a run's from the
+// replacements before it.  A whole separation at n = 343, T = 5000 takes 1.6 ms
+// instead of 46; what bounds the replay is the chunk's chain of CTA barriers
+// and the read of the candidates by one SM.
 #pragma once
 #include "trisep.cuh"
 
@@ -100,13 +103,13 @@ __device__ inline void tr_replay_warp(const TriCand* __restrict__ cand, long lon
 }
 
 // First position in the ascending a[0..n) whose value is >= x (GE) or > x.
-template <bool GE>
-__device__ __forceinline__ int tr_bound(const double* a, int n, double x)
+template <bool GE, class V>
+__device__ __forceinline__ int tr_bound(const V* a, int n, V x)
 {
     int lo = 0;
     for (int len = n; len > 0;) {
         const int half = len >> 1;
-        const double v = a[lo + half];
+        const V v = a[lo + half];
         const bool right = GE ? v < x : v <= x;
         lo = right ? lo + half + 1 : lo;
         len = right ? len - half - 1 : half;
@@ -139,9 +142,8 @@ __device__ __forceinline__ int tr_prefix(int v, int* ws, int* total)
 }
 
 // The replay, by a CTA of TR_THREADS threads (V > T > 0): list[slot] for every
-// slot.  Returns false (uniformly, list untouched) when equal values make the
-// order ambiguous.  sm: tr_smem_bytes(T) bytes of shared memory.
-__device__ inline bool tr_replay_cta(const TriCand* __restrict__ cand, long long V, int T,
+// slot.  sm: tr_smem_bytes(T) bytes of shared memory.
+__device__ inline void tr_replay_cta(const TriCand* __restrict__ cand, long long V, int T,
                                      TriCand* __restrict__ list, double* sm)
 {
     constexpr int S = TR_THREADS;
@@ -150,14 +152,14 @@ __device__ inline bool tr_replay_cta(const TriCand* __restrict__ cand, long long
     double* lw = lv + T;                  // (the other list's)
     double* xv = lw + T;                  // the chunk in arrival order
     double* mv = xv + S;                  // merge sort, 2 x S
-    double* ev = mv + 2 * S;              // removed values (S)
+    double* ev = mv + 2 * S;              // taken values, ascending (S)
     int* ls = (int*)(ev + S);             // slots,
     int* li = ls + T;                     // candidates
     int* lt = li + T;
     int* lj = lt + T;
     int* xi = lj + T;                     // candidates of the chunk
     int* mp = xi + S;                     // arrival positions, 2 x S
-    int* ep = mp + 2 * S;                 // by sorted position: taken ones before it
+    int* ep = mp + 2 * S;                 // equal values: a taken one's slot
     int* tk = ep + S;                     // by arrival position: rank among the taken, or -1
     int* rf = tk + S;                     // replacement t: a slot, or -1 - the replacement it follows
     int* rg = rf + S;
@@ -287,59 +289,131 @@ __device__ inline bool tr_replay_cta(const TriCand* __restrict__ cand, long long
         const bool staken = tid < n && tk[sp[tid < n ? tid : 0]] >= 0;
         int dummy;
         const int before = tr_prefix(staken ? 1 : 0, ws, &dummy);
-        ep[tid] = before;
-        __syncthreads();
         if (e == 0) continue;
-        // places in the union: list values first among equals
-        for (int q = tid; q < T; q += S) {
-            const double x = lv[q];
-            const int c = tr_bound<true>(sv, n, x);   // chunk values < x
-            const int p = q + (c < n ? ep[c] : e);
-            if (p < e) {
-                ev[p] = x;
-                rf[p] = ls[q];
-            } else {
-                lw[p - e] = x;
-                lt[p - e] = ls[q];
-                lj[p - e] = li[q];
-            }
-        }
-        int place = -1, event = -1;
+        // the taken ones in ascending order: place u = before; below: list values
+        // smaller than it
+        int event = -1, id = 0;
+        double x = 0.0;
+        bool equal = false;
         if (staken) {
             const int a = sp[tid];
+            x = sv[tid];
             event = tk[a];
-            const double x = sv[tid];
-            place = tr_bound<false>(lv, T, x) + before;
-            if (place < e) {
-                ev[place] = x;
-                rf[place] = -1 - event;
-            } else {
-                lw[place - e] = x;
-                lj[place - e] = xi[a];
-            }
+            id = xi[a];
+            below = tr_bound<true>(lv, T, x);
+            equal = below < T && lv[below] == x;
+            ev[before] = x;
         }
         __syncthreads();
-        // equal values among the removed ones, or with the new minimum
-        bool tie = false;
-        if (tid < e) tie = ev[tid] == (tid + 1 < e ? ev[tid + 1] : lw[0]);
-        if (__syncthreads_or(tie)) return false;
-        // replacement t takes the slot of what it removed (chains of up to S)
-        bool more = true;
-        for (int jump = 1; more && jump <= 2 * S; jump <<= 1) {
-            bool open = false;
-            if (tid < e) {
-                const int r = rf[tid];
-                const int s = r < 0 ? rf[-1 - r] : r;
-                rg[tid] = s;
-                open = s < 0;
+        if (staken) equal = equal || (before + 1 < e && ev[before + 1] == x);
+        if (!__syncthreads_or(equal)) {
+            // places in the union
+            for (int q = tid; q < T; q += S) {
+                const double y = lv[q];
+                const int p = q + tr_bound<true>(ev, e, y);
+                if (p < e) {
+                    rf[p] = ls[q];
+                } else {
+                    lw[p - e] = y;
+                    lt[p - e] = ls[q];
+                    lj[p - e] = li[q];
+                }
             }
-            more = __syncthreads_or(open) != 0;
-            int* t = rf;
-            rf = rg;
-            rg = t;
+            const int place = below + before;
+            if (staken) {
+                if (place < e) {
+                    rf[place] = -1 - event;
+                } else {
+                    lw[place - e] = x;
+                    lj[place - e] = id;
+                }
+            }
+            __syncthreads();
+            // replacement t takes the slot of what it removed (chains of up to S: at
+            // most ten doublings)
+            bool more = true;
+            for (int jump = 1; more && jump <= 2 * S; jump <<= 1) {
+                bool open = false;
+                if (tid < e) {
+                    const int r = rf[tid];
+                    const int s = r < 0 ? rf[-1 - r] : r;
+                    rg[tid] = s;
+                    open = s < 0;
+                }
+                more = __syncthreads_or(open) != 0;
+                int* t = rf;
+                rf = rg;
+                rg = t;
+            }
+            if (staken && place >= e) lt[place - e] = rf[event];
+        } else {
+            // (what the chunk's arrays held is in registers)
+            int* const cb = (int*)mv;   // by place u: list values smaller,
+            int* const ce = cb + S;     // smaller or equal,
+            int* const ue = ce + S;     // the end of its run of equal taken ones,
+            int* const ci = xi;         // its candidate;
+            int* const fs = mp;         // slots and candidates, a run by slots
+            int* const fi = mp + S;
+            if (staken) {
+                cb[before] = below;
+                ce[before] = tr_bound<false>(lv, T, x);
+                ue[before] = tr_bound<false>(ev, e, x);
+                rg[before] = event;
+                ci[before] = id;
+            }
+            // rf[t]: the slot that replacement t takes; first the list's values that
+            // no taken one equals
+            if (tid < T && tid < e) {
+                const double y = lv[tid];
+                const int u = tr_bound<true>(ev, e, y);
+                if (tid + u < e && !(u < e && ev[u] == y)) rf[tid + u] = ls[tid];
+            }
+            __syncthreads();
+            if (warp == 0) {
+                for (int u0 = 0; u0 < e;) {
+                    const int u1 = ue[u0], a = cb[u0], b = ce[u0];
+                    for (int u = u0 + lane; u < u1; u += 32) ep[u] = rf[rg[u]];
+                    __syncwarp();
+                    for (int u = u0 + lane; u < u1; u += 32) {
+                        int r = u0;
+                        for (int w = u0; w < u1; ++w) r += ep[w] < ep[u] ? 1 : 0;
+                        fs[r] = ep[u];
+                        fi[r] = ci[u];
+                    }
+                    __syncwarp();
+                    for (int u = u0 + lane; u < u1; u += 32) {
+                        const int p = a + u + tr_bound<true>(ls + a, b - a, fs[u]);
+                        if (p < e) rf[p] = fs[u];
+                    }
+                    for (int q = a + lane; q < b && q + u0 < e; q += 32) {
+                        const int p = q + u0 + tr_bound<true>(fs + u0, u1 - u0, ls[q]);
+                        if (p < e) rf[p] = ls[q];
+                    }
+                    __syncwarp();
+                    u0 = u1;
+                }
+            }
+            __syncthreads();
+            for (int q = tid; q < T; q += S) {
+                const double y = lv[q];
+                int u = tr_bound<true>(ev, e, y);
+                if (u < e && ev[u] == y) u += tr_bound<true>(fs + u, ue[u] - u, ls[q]);
+                const int p = q + u - e;
+                if (p >= 0) {
+                    lw[p] = y;
+                    lt[p] = ls[q];
+                    lj[p] = li[q];
+                }
+            }
+            if (tid < e) {
+                const int a = cb[tid], p = a + tid + tr_bound<true>(ls + a, ce[tid] - a, fs[tid]) - e;
+                if (p >= 0) {
+                    lw[p] = ev[tid];
+                    lt[p] = fs[tid];
+                    lj[p] = fi[tid];
+                }
+            }
         }
-        if (more) return false;
-        if (staken && place >= e) lt[place - e] = rf[event];
         __syncthreads();
         double* t = lv;
         lv = lw;
@@ -353,7 +427,6 @@ __device__ inline bool tr_replay_cta(const TriCand* __restrict__ cand, long long
     }
     for (int q = tid; q < T; q += S) list[ls[q]] = cand[li[q]];
     __syncthreads();
-    return true;
 }
 
 }  // namespace bqb
