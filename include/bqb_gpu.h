@@ -467,7 +467,8 @@ void bqb_ipm_schedule_set(int n, int grid);
  * off by default): out[8] = {ms waiting at grid barriers, ms in panel
  * factorisations, ms in tile updates, ms in the products, ms in whole
  * calls, grid barriers, sweep phases, ms of the panel factorisations
- * spent loading the panel block}; reset != 0 zeroes after reading.  For
+ * until the panel block has come (the first tile is loaded beside it)};
+ * reset != 0 zeroes after reading.  For
  * profiling; no reference counterpart. */
 void bqb_ipm_coop_profile_enable(int on);
 void bqb_ipm_coop_profile(double *out, int reset);

@@ -94,13 +94,13 @@ struct CoopArgs {
 // Parts of the time CTA 0 spends in a call (bqb_ipm_coop_profile).
 enum CoopProf : int {
     COOP_PROF_BARRIER,   // waiting at grid barriers
-    COOP_PROF_FACTOR,    // the panel factorisations (every CTA factors each panel block)
+    COOP_PROF_FACTOR,    // the panel factorisations (every CTA factors each panel block), its loads and the first tile's included
     COOP_PROF_TILES,     // the sweeps' tile updates
     COOP_PROF_GEMM,      // the two symmetric products
     COOP_PROF_TOTAL,     // the whole call
     COOP_PROF_BARRIERS,  // count of grid barriers
     COOP_PROF_PHASES,    // count of sweep phases
-    COOP_PROF_PF_LOAD,   // the part of the panel factorisations spent loading the panel block
+    COOP_PROF_PF_LOAD,   // the part of them until the panel block has come (trial 0's)
     COOP_PROF_WORDS = 8
 };
 
@@ -672,6 +672,10 @@ __device__ __noinline__ bool msweep(TrialSet& ts, const CoopArgs& a, Smem& sm)
         TileLoad load;
         int q = blockIdx.x;
         if (q < total) tile_load(addr, load);
+        if (rec && wrun) {   // (a use of the last pair, so that the clock is read after it)
+            *(volatile double*)sm.red = pf.d[3][3].y;
+            prof[COOP_PROF_PF_LOAD] += global_ns() - tp;
+        }
         if (wrun && w < NTRIAL) panel_chain(pf, wt, wfull, sm);
         if (wrun && w >= NTRIAL && wfull) panel_help(wt, sm);
         __syncthreads();
@@ -1434,7 +1438,8 @@ BQB_API int bqb_ipm_autotune(int n, int reps, int* best_grid, double* best_ms)
 // Time the multi-CTA IPM spends per part (its CTA 0, summed over calls since
 // the last reset): enable (on != 0) or disable the timing; out[8] = {barrier
 // waits, panel factorisations, tile updates, products, whole calls (ms),
-// grid barriers, sweep phases, the panel factorisations' block loads (ms)};
+// grid barriers, sweep phases, the part of the panel factorisations until the
+// panel block has come (ms)};
 // reset != 0 zeroes after reading.  For
 // profiling; no reference counterpart.
 BQB_API void bqb_ipm_coop_profile_enable(int on) { g_coop_prof_on.store(on != 0); }
