@@ -66,10 +66,10 @@ WORKLOAD = "G(100,0.5) ±1 weights; 512 subproblems, k~U[0,40] fixed (n=60..100)
 FLOP_PER_ITER_N3 = 6.0
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the fused
 # kernel per node, from one ncu capture of a 512-node launch of this workload
-# (1.85 GB read + 3.97 GB written, 1 pass); the line reports it scaled to the
+# (0.77 GB read + 1.38 GB written, 1 pass); the line reports it scaled to the
 # average nodes per launch.
-NODEK_DRAM_BYTES_PER_NODE = (1.85e9 + 3.97e9) / 512
-NODEK_TRAFFIC_NOTE = ("ncu capture of one 512-node launch of this workload (1.85 GB read + 3.97 GB written), "
+NODEK_DRAM_BYTES_PER_NODE = (0.769e9 + 1.384e9) / 512
+NODEK_TRAFFIC_NOTE = ("ncu capture of one 512-node launch of this workload (0.77 GB read + 1.38 GB written), "
                       "scaled to the average nodes per launch")
 FP64_NOMINAL_TFLOPS = 37.0
 
@@ -590,9 +590,10 @@ def run_gpu(args):
             "traffic": NODEK_DRAM_BYTES_PER_NODE * int(fst[0]) * B / max(n_launch, 1),
             "traffic_note": NODEK_TRAFFIC_NOTE,
             "peak_source": f"{pk['source']} bf16 sustained (the contract's compute denominator); the kernel "
-                           "computes in FP64 on the CUDA cores (no tensor-core instruction), so its own ceiling "
+                           "computes in FP64 (the IPM's tiles with mma.sync m8n8k4 f64, the rest on the CUDA "
+                           "cores; tcgen05 has no FP64 form), so its own ceiling "
                            f"is B200's nominal FP64 37 TFLOP/s: frac of that {achieved / FP64_NOMINAL_TFLOPS:.4f}",
-            "pipe": "fp64 (CUDA cores)", "frac_of_fp64_nominal": achieved / FP64_NOMINAL_TFLOPS,
+            "pipe": "fp64 (tensor instruction and CUDA cores)", "frac_of_fp64_nominal": achieved / FP64_NOMINAL_TFLOPS,
             "achieved_over": "span of the pipelined launches (CUDA events on the idle current stream around "
                              "every submission and collection)",
             "launches": n_launch, "submissions": int(fst[0]), "span_ms": span_ms,
