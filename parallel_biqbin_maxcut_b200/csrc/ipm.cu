@@ -284,12 +284,30 @@ ipm_reg_one_kernel(IpmDesc d, int smem_doubles)
     ipm_body_reg(d, smem_doubles, g_ipm_stats);
 }
 
+// n <= 8 (a kernel of its own: as a branch of the one above it cost n = 24 four
+// per cent)
+__global__ void __launch_bounds__(IPM_THREADS, 1)
+ipm_reg_tile_kernel(IpmDesc d, int smem_doubles)
+{
+    if (d.n <= 0) return;
+    ipm_body_reg<true>(d, smem_doubles, g_ipm_stats);
+}
+
 __global__ void __launch_bounds__(IPM_THREADS, 1)
 ipm_reg_batched_kernel(const IpmDesc* __restrict__ descs, int smem_doubles)
 {
     const IpmDesc d = descs[blockIdx.x];
     if (d.n <= 0) return;
     ipm_body_reg(d, smem_doubles, g_ipm_stats);
+}
+
+// (n <= 8)
+__global__ void __launch_bounds__(IPM_THREADS, 1)
+ipm_reg_tile_batched_kernel(const IpmDesc* __restrict__ descs, int smem_doubles)
+{
+    const IpmDesc d = descs[blockIdx.x];
+    if (d.n <= 0) return;
+    ipm_body_reg<true>(d, smem_doubles, g_ipm_stats);
 }
 
 __global__ void __launch_bounds__(IPM_THREADS, 1)
@@ -420,8 +438,9 @@ void ipm_launch(const IpmDesc* d_descs, int nprob, int n_max, cudaStream_t s)
     if (n_max <= ST_NMAX) {
         const int sd = ipm_reg_smem(n_max);
         bytes = sd * sizeof(double);
-        BQB_SMEM_LIMIT(ipm_reg_batched_kernel, bytes);
-        t_timer.timed(s, [&] { ipm_reg_batched_kernel<<<nprob, IPM_THREADS, bytes, s>>>(d_descs, sd); });
+        auto* kernel = n_max <= 8 ? ipm_reg_tile_batched_kernel : ipm_reg_batched_kernel;
+        BQB_SMEM_LIMIT(kernel, bytes);
+        t_timer.timed(s, [&] { kernel<<<nprob, IPM_THREADS, bytes, s>>>(d_descs, sd); });
         BQB_COUNT_LAUNCH();
         check_launch("ipm_reg_batched_kernel");
         return;
@@ -439,8 +458,9 @@ void ipm_launch_one(const IpmDesc& d, cudaStream_t s)
     if (d.n <= ST_NMAX) {
         const int sd = ipm_reg_smem(d.n);
         bytes = sd * sizeof(double);
-        BQB_SMEM_LIMIT(ipm_reg_one_kernel, bytes);
-        t_timer.timed(s, [&] { ipm_reg_one_kernel<<<1, IPM_THREADS, bytes, s>>>(d, sd); });
+        auto* kernel = d.n <= 8 ? ipm_reg_tile_kernel : ipm_reg_one_kernel;
+        BQB_SMEM_LIMIT(kernel, bytes);
+        t_timer.timed(s, [&] { kernel<<<1, IPM_THREADS, bytes, s>>>(d, sd); });
         BQB_COUNT_LAUNCH();
         check_launch("ipm_reg_one_kernel");
         return;
@@ -454,9 +474,10 @@ void ipm_launch_one(const IpmDesc& d, cudaStream_t s)
 cudaError_t ipm_launch_prepared(const IpmDesc& d, size_t smem_limit, cudaStream_t s)
 {
     const size_t sd = ipm_st_smem_doubles(d.n, smem_limit / sizeof(double));
-    cudaError_t e = raise_smem_limit((const void*)ipm_reg_one_kernel, sd * sizeof(double));
+    auto* kernel = d.n <= 8 ? ipm_reg_tile_kernel : ipm_reg_one_kernel;
+    cudaError_t e = raise_smem_limit((const void*)kernel, sd * sizeof(double));
     if (e != cudaSuccess) return e;
-    ipm_reg_one_kernel<<<1, IPM_THREADS, sd * sizeof(double), s>>>(d, (int)sd);
+    kernel<<<1, IPM_THREADS, sd * sizeof(double), s>>>(d, (int)sd);
     BQB_COUNT_LAUNCH();
     return cudaGetLastError();
 }

@@ -114,17 +114,18 @@ __device__ __forceinline__ double2 ipm_st_z(const IpmSt& s, double al, int I, in
 }
 
 // Zi = inv(Z + al Diag(dy)) (not inlined, nor the others here: the tiles in
-// registers then have the whole register budget).
+// registers then have the whole register budget).  ONE: of one tile.
+template <bool ONE>
 static __device__ __noinline__ bool ipm_st_inv_z(const IpmSt& s, double al)
 {
     const int T = s.T, lane = threadIdx.x & 31;
     double* Zi = s.Zi();
-    if (T < 16)
-        return st_inverse(
-            T, s.buf(), s.flag(), [&](int I, int J, int r, int c) { return ipm_st_z(s, al, I, J, r, c); },
-            [&](int I, int J, double a, double b) {
-                st_st(Zi + 64 * (I * T + J) + st_pair(lane >> 2, lane & 3), a, b);
-            });
+    auto fill = [&](int I, int J, int r, int c) { return ipm_st_z(s, al, I, J, r, c); };
+    auto store = [&](int I, int J, double a, double b) {
+        st_st(Zi + 64 * (I * T + J) + st_pair(lane >> 2, lane & 3), a, b);
+    };
+    if constexpr (ONE) return st_inverse_one(s.n, fill, store);
+    if (T < 16) return st_inverse(T, s.buf(), s.flag(), fill, store);
     RegMat R;
     const int n = s.n;
     rm_fill(R, n, [&](int r, int c) { return r == c ? fma(al, s.dy()[r], s.zd()[r]) : -s.L[r + (size_t)c * n]; });
@@ -140,28 +141,28 @@ static __device__ __noinline__ bool ipm_st_inv_z(const IpmSt& s, double al)
 }
 
 // F = inv(Zi .* X)
+template <bool ONE>
 static __device__ __noinline__ bool ipm_st_inv_m(const IpmSt& s)
 {
     const int T = s.T, n = s.n, lane = threadIdx.x & 31;
     const double* X = s.X();
     const double* Zi = s.Zi();
     double* F = s.F;
-    if (T < 16)
-        return st_inverse(
-            T, s.buf(), s.flag(),
-            [&](int I, int J, int r, int c) {
-                const int i = 8 * I + r, j = 8 * J + 2 * c;
-                const double2 z = st_ld(Zi + 64 * (I * T + J) + st_pair(r, c));
-                double2 v = make_double2(i == j ? 1.0 : 0.0, i == j + 1 ? 1.0 : 0.0);
-                if (i < n && j < n) v.x = z.x * X[IpmSt::sym(i, j)];
-                if (i < n && j + 1 < n) v.y = z.y * X[IpmSt::sym(i, j + 1)];
-                return v;
-            },
-            [&](int I, int J, double a, double b) {
-                double* f = F + 8 * I + (lane >> 2) + (size_t)(8 * J + 2 * (lane & 3)) * (8 * T);
-                f[0] = a;
-                f[8 * T] = b;
-            });
+    auto fill = [&](int I, int J, int r, int c) {
+        const int i = 8 * I + r, j = 8 * J + 2 * c;
+        const double2 z = st_ld(Zi + 64 * (I * T + J) + st_pair(r, c));
+        double2 v = make_double2(i == j ? 1.0 : 0.0, i == j + 1 ? 1.0 : 0.0);
+        if (i < n && j < n) v.x = z.x * X[IpmSt::sym(i, j)];
+        if (i < n && j + 1 < n) v.y = z.y * X[IpmSt::sym(i, j + 1)];
+        return v;
+    };
+    auto store = [&](int I, int J, double a, double b) {
+        double* f = F + 8 * I + (lane >> 2) + (size_t)(8 * J + 2 * (lane & 3)) * (8 * T);
+        f[0] = a;
+        f[8 * T] = b;
+    };
+    if constexpr (ONE) return st_inverse_one(n, fill, store);
+    if (T < 16) return st_inverse(T, s.buf(), s.flag(), fill, store);
     RegMat R;
     rm_fill(R, n, [&](int r, int c) { return Zi[s.all(r, c)] * X[IpmSt::sym(r, c)]; });
     const bool pd = rm_spd_inverse(R, n, s.buf());
@@ -171,11 +172,12 @@ static __device__ __noinline__ bool ipm_st_inv_m(const IpmSt& s)
 }
 
 // X + al dX (Z + al Diag(dy) with dual) positive definite?
+template <bool ONE>
 static __device__ __noinline__ bool ipm_st_trial(const IpmSt& s, bool dual, double al)
 {
     const double* X = s.X();
     const double* Q = s.Q;
-    return st_posdef(s.T, s.buf(), s.flag(), [&](int I, int J, int r, int c) {
+    auto fill = [&](int I, int J, int r, int c) {
         double2 v;
         if (dual) {
             v = ipm_st_z(s, al, I, J, r, c);
@@ -186,7 +188,9 @@ static __device__ __noinline__ bool ipm_st_trial(const IpmSt& s, bool dual, doub
             if (I == J && 8 * I + r >= s.n) v = make_double2(r == 2 * c ? 1.0 : 0.0, r == 2 * c + 1 ? 1.0 : 0.0);
         }
         return make_double2(-v.x, -v.y);
-    });
+    };
+    if constexpr (ONE) return st_posdef_one(s.n, fill);
+    return st_posdef(s.T, s.buf(), s.flag(), fill);
 }
 
 // out = F v, one warp per row, reading F's column (v null: v = -e); four rows
@@ -339,7 +343,9 @@ static __device__ __noinline__ void ipm_st_corrector(const IpmSt& s, double mu, 
 
 // stats (optional, device): the work counters [iterations n^3, problems,
 // iterations, line-search trials] are added there.  smem_doubles: the CTA's
-// dynamic shared memory (st_smem).
+// dynamic shared memory (st_smem).  ONE: for n <= 8 only, by one warp's
+// eliminations.
+template <bool ONE = false>
 __device__ inline void ipm_body_reg(const IpmDesc& d, int smem_doubles, double* stats)
 {
     const int tid = threadIdx.x;
@@ -419,11 +425,11 @@ __device__ inline void ipm_body_reg(const IpmDesc& d, int smem_doubles, double* 
         if (++iter > IPM_MAX_ITERS) { status = IPM_MAXITER; break; }
 
         // ---- Zi = inv(Z), Z = Diag(zd) - L off the diagonal ----
-        if (!have_zi && !ipm_st_inv_z(s, 0.0)) { status = IPM_Z_NOT_PD; break; }
+        if (!have_zi && !ipm_st_inv_z<ONE>(s, 0.0)) { status = IPM_Z_NOT_PD; break; }
         have_zi = false;
         // ---- F = inv(M), M = Zi .* X; dy1 = M \ (-e) (a non-positive pivot of
         // M is where the reference's dposv fails) ----
-        if (!ipm_st_inv_m(s)) { status = IPM_M_NOT_PD; break; }
+        if (!ipm_st_inv_m<ONE>(s)) { status = IPM_M_NOT_PD; break; }
         ipm_st_apply(s, nullptr, dy1);
 
         // ---- dX1 = sym(Zi (-Diag(dy1) X) - X) ----
@@ -454,7 +460,7 @@ __device__ inline void ipm_body_reg(const IpmDesc& d, int smem_doubles, double* 
         int trials = 0;
         bool ok = false;
         while (true) {
-            if (ipm_st_trial(s, false, ap)) { ok = true; break; }
+            if (ipm_st_trial<ONE>(s, false, ap)) { ok = true; break; }
             if (++trials >= IPM_MAX_TRIALS) break;
             ap *= 0.8;
         }
@@ -467,7 +473,7 @@ __device__ inline void ipm_body_reg(const IpmDesc& d, int smem_doubles, double* 
         trials = 0;
         ok = false;
         while (true) {
-            if (trials == 0 ? ipm_st_inv_z(s, ad) : ipm_st_trial(s, true, ad)) { ok = true; break; }
+            if (trials == 0 ? ipm_st_inv_z<ONE>(s, ad) : ipm_st_trial<ONE>(s, true, ad)) { ok = true; break; }
             if (++trials >= IPM_MAX_TRIALS) break;
             ad *= 0.8;
         }

@@ -163,8 +163,10 @@ __device__ __forceinline__ void st_eliminate(double2& t, const double* mult, con
 // for the other warps: the multipliers u_q inv by steps, the operand of the
 // panel's own row (its row i starts at step i with the multipliers and takes
 // the later steps: 0 before, 1 at and -u_i after step i), the block, the
-// reciprocals.  False on a non-positive pivot, in every lane.
-__device__ __forceinline__ bool st_diagonal(double2 d, double* set)
+// reciprocals.  False on a non-positive pivot, in every lane.  ALONE: the first
+// n steps of a matrix's only tile, with nothing left in set.
+template <bool ALONE = false>
+__device__ __forceinline__ bool st_diagonal(double2& d, double* set, int n = 8)
 {
     const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
     const int row0 = lane & ~3;
@@ -174,6 +176,7 @@ __device__ __forceinline__ bool st_diagonal(double2 d, double* set)
     double p = __shfl_sync(ALL, d.x, 0);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+        if (ALONE && j >= n) break;
         const int h = j >> 1;
         const double dj = (j & 1) ? d.y : d.x;
         double e = 0.0, pn = 1.0;
@@ -193,6 +196,7 @@ __device__ __forceinline__ bool st_diagonal(double2 d, double* set)
         const double a0 = fma(-dr, w0, d.x), a1 = fma(-dr, w1, d.y);
         d.x = 2 * c == j ? (r == j ? -inv : dv) : (r == j ? w0 : a0);
         d.y = 2 * c + 1 == j ? (r == j ? -inv : dv) : (r == j ? w1 : a1);
+        if (ALONE) continue;
         if (r == j) st_st(set + 8 * j + 2 * c, w0, w1);
         if (c == (j & 3)) {
             const double v = r == j ? 1.0 : (r < j ? -dr : 0.0);
@@ -201,6 +205,7 @@ __device__ __forceinline__ bool st_diagonal(double2 d, double* set)
         }
         if (lane == 0) set[192 + j] = inv;
     }
+    if (ALONE) return pd;
     const StOp op;
     set[64 + op.o] = po.x;
     set[64 + op.o + op.d] = po.y;
@@ -356,9 +361,9 @@ __device__ __forceinline__ bool st_inverse(int T, double* buf, int* flag, Fill f
 // pivot's reciprocal square root is computed, and every lane computes the next
 // pivot for itself, so the chain is eight times a reciprocal square root, a
 // product and an FMA (69 + 8 + 8 cycles) and no shuffle is in it.  WITH_L: L
-// itself, too.
-template <bool WITH_L = false>
-__device__ __forceinline__ bool st_chol_inv(double2 d, double2& y, double2* l = nullptr)
+// itself, too.  ALONE: the first n steps of a matrix's only tile.
+template <bool WITH_L = false, bool ALONE = false>
+__device__ __forceinline__ bool st_chol_inv(double2 d, double2& y, double2* l = nullptr, int n = 8)
 {
     const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
     const int row0 = lane & ~3;
@@ -368,6 +373,7 @@ __device__ __forceinline__ bool st_chol_inv(double2 d, double2& y, double2* l = 
     double p = __shfl_sync(ALL, d.x, 0);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+        if (ALONE && j >= n) break;
         const int h = j >> 1;
         const double dj = (j & 1) ? d.y : d.x;
         double e = 0.0, pn = 1.0;
@@ -520,6 +526,43 @@ __device__ __forceinline__ bool st_posdef(int T, double* buf, int* flag, Fill fi
         if (!stopped) st_bar_sync(ST_BAR_L + ((T - 1) & 1), NC);
     }
     return __syncthreads_or(failed) == 0;
+}
+
+// ---- matrices of one tile (n <= 8) ---------------------------------------------
+//
+// One warp takes the n steps, without roles and their hand-overs and without the
+// padding's steps, which a bound of a few vertices would spend most of its time
+// in: n = 1, 2, 4, 8 took 105, 106, 143, 144 us with st_inverse and st_posdef (73,
+// 82, 144, 196 with single columns) and take 57, 57, 73, 82.  The same bits.
+
+// As st_inverse.
+template <class Fill, class Store>
+__device__ __forceinline__ bool st_inverse_one(int n, Fill fill, Store store)
+{
+    const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
+    __syncthreads();
+    bool pd = true;
+    if (threadIdx.x < 32) {
+        double2 d = fill(0, 0, r, c);
+        pd = st_diagonal<true>(d, nullptr, n);
+        store(0, 0, r < n ? -d.x : d.x, r < n ? -d.y : d.y);   // (the identity outside)
+    }
+    return __syncthreads_and(pd) != 0;
+}
+
+// As st_posdef (nothing is stored).
+template <class Fill>
+__device__ __forceinline__ bool st_posdef_one(int n, Fill fill)
+{
+    const int lane = threadIdx.x & 31;
+    __syncthreads();
+    bool pd = true;
+    if (threadIdx.x < 32) {
+        const double2 d = fill(0, 0, lane >> 2, lane & 3);
+        double2 y;
+        pd = st_chol_inv<false, true>(make_double2(-d.x, -d.y), y, nullptr, n);
+    }
+    return __syncthreads_and(pd) != 0;
 }
 
 // The Cholesky factor of the n x n matrix A (column-major, n <= 128, lower
