@@ -16,6 +16,10 @@ from test_zz_no_alloc import _noalloc, _regular
 
 @pytest.fixture(scope="module")
 def inverse(lib, tmp_path_factory):
+    try:
+        build.nvcc()
+    except RuntimeError:
+        pytest.skip("no nvcc to build tests/inverse_bits.cu with")
     so = str(tmp_path_factory.mktemp("inverse") / "inverse_bits.so")
     src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "inverse_bits.cu")
     subprocess.run([build.nvcc()] + build.NVCC_FLAGS + ["-I" + build.CSRC, "-shared", "-o", so, src], check=True)

@@ -1,7 +1,7 @@
 """The grid that the multi-CTA IPM (n > 128) uses without a schedule's entry is
 the fastest: no other, of the autotuner's candidates or a CTA for half a pair of
 32 x 32 tiles, is faster by more than the timing's spread (1.5 %; the best of
-12 calls of one grid, taken in turn with the others', repeats to 0.3 %)."""
+24 calls of one grid, taken in turn with the others', repeats to 0.3 %)."""
 import ctypes as C
 import time
 
@@ -20,7 +20,7 @@ def test_default_grid_is_the_fastest(lib, n):
     T = (n + 31) // 32
     best = {g: 1e9 for g in (0, 148, T * T, T * (T + 1), (T * T + 1) // 2)}   # (0: no entry)
     try:
-        for _ in range(12):
+        for _ in range(24):
             for g in best:
                 lib.bqb_ipm_schedule_set(n, g)
                 t = time.perf_counter()
