@@ -1245,8 +1245,7 @@ unsigned long long* coop_prof_device()
 
 // The per-size schedule: the grid (CTAs) to use for T = ceil(n / 32) tiles
 // per dimension, filled by the autotuner (bqb_ipm_autotune) or set by hand
-// (bqb_ipm_schedule_set); sizes without an entry use every CTA that can be
-// co-resident.
+// (bqb_ipm_schedule_set); sizes without an entry use coop_config's rule.
 std::mutex g_sched_mu;
 std::map<int, int> g_sched;
 
@@ -1260,15 +1259,10 @@ std::atomic<int> g_large_share{0};
 
 namespace {
 
-// Grid size for n: the schedule's entry for its tile count, else as many CTAs
-// as can be co-resident (one per SM at this register count); divided by the
-// number of engines bounding large nodes at the time.  The whole chip is the
-// fastest grid from n = 129 to 384, although a phase of a small problem has fewer
-// tiles than CTAs (the line searches sweep up to four matrices together, and
-// the fills and the products have more parts than tiles).  Microseconds a call
-// with a CTA for half a tile pair (T (T + 1) of them) and with 148: n = 136 1557,
-// 1518; 160 1917, 1859; 192 2225, 2176; 224 2429, 2373; 256 2399, 2326; 288 2853,
-// 2818; 320 3180, 3164; 343 4143, 4142.
+// Grid size for n: the schedule's entry for its tile count, else one CTA for
+// half a pair of 32 x 32 tiles (and the whole chip from 7/8 of it on); at most as many as can be co-resident (one
+// per SM at this register count), divided by the number of engines bounding
+// large nodes at the time.
 CoopConfig coop_config(int n)
 {
     static int max_blocks = -1;
@@ -1283,7 +1277,7 @@ CoopConfig coop_config(int n)
         ready.store(1);
     }
     const int T = (n + CB - 1) / CB;
-    int g = max_blocks;
+    int g = 8 * T * (T + 1) >= 7 * max_blocks ? max_blocks : T * (T + 1);
     {
         std::lock_guard<std::mutex> lock(g_sched_mu);
         auto it = g_sched.find(T);
@@ -1365,10 +1359,10 @@ BQB_API void bqb_ipm_schedule_set(int n, int grid)
 }
 
 // Autotune the multi-CTA IPM's grid for size n (> 128): time `reps` calls
-// for each candidate (the SM count, which is what a size without an entry
-// uses, and T^2 CTAs, T = ceil(n / 32), a half, a quarter and an eighth of that)
-// on a seeded problem of that size (the Laplacian of a random +-1 graph, as the
-// B&B's subproblems are), keep the fastest in the schedule.  best_grid / best_ms (may be null) receive the choice and its
+// for each candidate (one CTA per tile, half, a quarter, an eighth, and the
+// SM count) on a seeded problem of that size (the Laplacian of a random
+// +-1 graph, as the B&B's subproblems are), keep the fastest in the
+// schedule.  best_grid / best_ms (may be null) receive the choice and its
 // time per call.  Returns 0, 1 for n <= 128.  No reference counterpart.
 BQB_API int bqb_ipm_autotune(int n, int reps, int* best_grid, double* best_ms)
 {
@@ -1401,11 +1395,11 @@ BQB_API int bqb_ipm_autotune(int n, int reps, int* best_grid, double* best_ms)
     dX.ensure(nn);
     out.ensure(4);
     const int T = (n + CB - 1) / CB;
-    std::vector<int> cand = {R.num_sms, T * T, (T * T + 1) / 2, (T * T + 3) / 4, (T * T + 7) / 8};
+    std::vector<int> cand = {T * T, (T * T + 1) / 2, (T * T + 3) / 4, (T * T + 7) / 8, R.num_sms};
     cudaEvent_t e0, e1;
     BQB_CUDA(cudaEventCreate(&e0));
     BQB_CUDA(cudaEventCreate(&e1));
-    int bg = R.num_sms;
+    int bg = T * T;
     double bms = 1e300;
     for (int g : cand) {
         if (g < 1) continue;
