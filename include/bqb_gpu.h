@@ -457,10 +457,12 @@ int bqb_ipm_batch_device(const double *const *Ls, double *const *Xs, const int *
 
 /* Per-size schedule of the multi-CTA IPM (n > 128, one cooperative launch
  * per call): bqb_ipm_schedule_set uses `grid` CTAs for every n with the
- * same number of 32-column panels (grid <= 0: back to one CTA per 32 x 32
- * tile).  bqb_ipm_autotune times `reps` calls for each candidate grid on a
- * seeded problem of size n and keeps the fastest (best_grid / best_ms may
- * be NULL); returns 0, 1 for n <= 128.  No reference counterpart. */
+ * same number of 32-column panels (grid <= 0: back to the default, one CTA
+ * for half a pair of 32 x 32 tiles, at most one per SM).  bqb_ipm_autotune
+ * times `reps` calls (at least three) alone for each candidate grid, the
+ * default among them, on a seeded problem of size n and keeps the one with
+ * the fastest call (best_grid / best_ms may be NULL); returns 0, 1 for n <=
+ * 128.  No reference counterpart. */
 void bqb_ipm_schedule_set(int n, int grid);
 /* Timing of the multi-CTA IPM by parts (its first CTA, summed over calls;
  * off by default): out[8] = {ms waiting at grid barriers, ms in panel

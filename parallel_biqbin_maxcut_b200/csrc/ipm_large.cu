@@ -1259,10 +1259,22 @@ std::atomic<int> g_large_share{0};
 
 namespace {
 
-// Grid size for n: the schedule's entry for its tile count, else one CTA for
-// half a pair of 32 x 32 tiles (and the whole chip from 7/8 of it on); at most as many as can be co-resident (one
-// per SM at this register count), divided by the number of engines bounding
-// large nodes at the time.
+// CTAs for T tiles per dimension: one for half a pair of 32 x 32 tiles, at most
+// max_blocks.  A call alone is faster with the whole chip (the line searches sweep
+// up to four matrices, and fills and products have more parts than tiles), by
+// 38 of 1557 us at n = 136, 58 of 1917 at 160, 56 of 2429 at 224, 35 of 2853 at 288,
+// nothing from 321 on; but a cooperative launch waits until all its CTAs find a
+// free SM, so beside other engines' one-CTA kernels the whole chip loses: eight
+// nodes of n = 130 on four engines take 59 ms so and 89 with it, of n = 200 53.8
+// and 54.7.
+int coop_default_grid(int T, int max_blocks)
+{
+    return T * (T + 1) < max_blocks ? T * (T + 1) : max_blocks;
+}
+
+// Grid size for n: the schedule's entry for its tile count, else the default; at
+// most as many as can be co-resident (one per SM at this register count),
+// divided by the number of engines bounding large nodes at the time.
 CoopConfig coop_config(int n)
 {
     static int max_blocks = -1;
@@ -1277,7 +1289,7 @@ CoopConfig coop_config(int n)
         ready.store(1);
     }
     const int T = (n + CB - 1) / CB;
-    int g = 8 * T * (T + 1) >= 7 * max_blocks ? max_blocks : T * (T + 1);
+    int g = coop_default_grid(T, max_blocks);
     {
         std::lock_guard<std::mutex> lock(g_sched_mu);
         auto it = g_sched.find(T);
@@ -1358,16 +1370,18 @@ BQB_API void bqb_ipm_schedule_set(int n, int grid)
     else g_sched.erase(T);
 }
 
-// Autotune the multi-CTA IPM's grid for size n (> 128): time `reps` calls
-// for each candidate (one CTA per tile, half, a quarter, an eighth, and the
-// SM count) on a seeded problem of that size (the Laplacian of a random
-// +-1 graph, as the B&B's subproblems are), keep the fastest in the
-// schedule.  best_grid / best_ms (may be null) receive the choice and its
-// time per call.  Returns 0, 1 for n <= 128.  No reference counterpart.
+// Autotune the multi-CTA IPM's grid for size n (> 128): time `reps` calls (at
+// least three) for each candidate (the default grid, T^2 CTAs, T = ceil(n / 32), a
+// half, a quarter and an eighth of that, and the SM count) on a seeded problem of
+// that size (the Laplacian of a random +-1 graph, as the B&B's subproblems are),
+// keep the one with the fastest call in the schedule.  best_grid / best_ms (may
+// be null) receive the choice and that time.  Calls are timed alone: beside other
+// engines a smaller grid may be better (coop_default_grid).  Returns 0, 1 for n <=
+// 128.  No reference counterpart.
 BQB_API int bqb_ipm_autotune(int n, int reps, int* best_grid, double* best_ms)
 {
     if (n <= 128) return 1;
-    if (reps < 1) reps = 1;
+    if (reps < 3) reps = 3;
     Runtime& R = rt();
     cudaStream_t s = R.stream;
     const size_t nn = (size_t)n * n;
@@ -1395,26 +1409,31 @@ BQB_API int bqb_ipm_autotune(int n, int reps, int* best_grid, double* best_ms)
     dX.ensure(nn);
     out.ensure(4);
     const int T = (n + CB - 1) / CB;
-    std::vector<int> cand = {T * T, (T * T + 1) / 2, (T * T + 3) / 4, (T * T + 7) / 8, R.num_sms};
+    const int def = coop_default_grid(T, R.num_sms);
+    std::vector<int> cand = {def, T * T, (T * T + 1) / 2, (T * T + 3) / 4, (T * T + 7) / 8, R.num_sms};
     cudaEvent_t e0, e1;
     BQB_CUDA(cudaEventCreate(&e0));
     BQB_CUDA(cudaEventCreate(&e1));
-    int bg = T * T;
+    int bg = def;
     double bms = 1e300;
     for (int g : cand) {
         if (g < 1) continue;
         bqb_ipm_schedule_set(n, g);
         ipm_large(ws, dL.p, dX.p, n, out.p, s, nullptr);   // warm-up
-        BQB_CUDA(cudaEventRecord(e0, s));
-        for (int r = 0; r < reps; ++r) ipm_large(ws, dL.p, dX.p, n, out.p, s, nullptr);
-        BQB_CUDA(cudaEventRecord(e1, s));
-        BQB_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        BQB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        float ms = 1e30f;
+        for (int r = 0; r < reps; ++r) {
+            float t = 0.f;
+            BQB_CUDA(cudaEventRecord(e0, s));
+            ipm_large(ws, dL.p, dX.p, n, out.p, s, nullptr);
+            BQB_CUDA(cudaEventRecord(e1, s));
+            BQB_CUDA(cudaEventSynchronize(e1));
+            BQB_CUDA(cudaEventElapsedTime(&t, e0, e1));
+            ms = t < ms ? t : ms;
+        }
         double h[4];
         BQB_CUDA(cudaMemcpy(h, out.p, sizeof h, cudaMemcpyDeviceToHost));
-        if ((int)h[2] == IPM_OK && ms / reps < bms) {
-            bms = ms / reps;
+        if ((int)h[2] == IPM_OK && ms < bms) {
+            bms = ms;
             bg = g;
         }
     }
