@@ -52,6 +52,18 @@ def test_equal_values(lib, rising, levels, T):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("levels", [0, 8])
+@pytest.mark.parametrize("n", [6, 10, 16, 20, 22, 24, 30])
+@pytest.mark.parametrize("T", [1, 2, 7, 8, 9])
+def test_short_lists(lib, n, levels, T):
+    X = _X(n, levels, False)
+    got, mx = gpu_sep(lib, X, T, 0.05)
+    want, mx_ref = O.getViolated_TriangleInequalities(X, T, 0.05)
+    assert mx == mx_ref
+    assert got == want
+
+
+@pytest.mark.gpu
 def test_equal_values_cost_no_replay_by_single_cuts(lib):
     """A list too long for shared memory is replayed one cut at a time; equal
     values in a shorter one take less than half of that."""
