@@ -155,7 +155,7 @@ double heuristic_device(HeurState& st, Rng& rng, const double* dX, const double*
         double v = heur_val;
         if (hyperplanes > 0 || abort_returns()) {
             // Draws cannot be taken back: a caller that lives on after a failed
-            // factorisation finds rand() where it stood before this round.
+            // factorisation finds rand() where the reference leaves it.
             BQB_CUDA(cudaMemcpyAsync(st.hstat.p, st.status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
             BQB_CUDA(cudaStreamSynchronize(s));
             ok = st.hstat.p[0] == 0;
